@@ -775,6 +775,8 @@ void admm_free(cdlgb_ctx* c) {
         if (c->hscalar_own) cudaFreeHost(c->hscalar);
         else host_scalars_put(c->hscalar);
     }
+    xconv_plan_free(c, c->xconv);
+    c->xconv = nullptr;
     dev_free(c, c->dres);
     dev_free(c, c->rpart);
     dev_free(c, c->Gprev);
@@ -901,12 +903,13 @@ int admm_code_update(cdlgb_ctx* c, int iters) {
     cudaStream_t s = c->stream;
     const size_t LN = c->LN;
     const int F = c->F, M = c->M, N = c->N;
-    if (iters > 0 && c->fused && fused_has_multi(c)) {
+    if (iters > 0 && (c->xconv || (c->fused && fused_has_multi(c)))) {
         // all iterations in one launch, the state on chip in between
         cdlgb_phase_begin(c, PH_XSTEP);
         float* Xin = cur_X(c);
         float* Xout = c->best_is_cur ? c->Xb[1 - c->xcur] : Xin;
-        ST_TRY(fused_xsteps(c, Xin, Xout, iters));
+        if (c->xconv) ST_TRY(xconv_xsteps(c, c->xconv, Xin, Xout, iters, c->N));
+        else ST_TRY(fused_xsteps(c, Xin, Xout, iters));
         c->absx_fused = 1;
         if (Xout != Xin) {
             c->xcur = 1 - c->xcur;
@@ -916,7 +919,7 @@ int admm_code_update(cdlgb_ctx* c, int iters) {
         const double* rp = nullptr;
         int nr = 0;
         if (c->res_on) {
-            if (fused_resid(c, &rp, &nr)) ST_TRY(resid_x_from_parts(c, rp, nr));
+            if (!c->xconv && fused_resid(c, &rp, &nr)) ST_TRY(resid_x_from_parts(c, rp, nr));
             else ST_TRY(resid_x_from_arrays(c, cur_X(c)));
         }
         cdlgb_phase_end_n(c, PH_XSTEP, iters);
@@ -1094,7 +1097,7 @@ static int objective_async(cdlgb_ctx* c) {
     if (c->absx_init) {
         // sum |X| came with the initial X (k_init_x)
         c->absx_init = 0;
-    } else if (c->absx_fused && fused_absx(c, &fp, &nf)) {
+    } else if (c->absx_fused && (c->xconv ? xconv_absx(c->xconv, &fp, &nf) : fused_absx(c, &fp, &nf))) {
         // sum |X| came with the last fused X-step
         pa = fp;
         nb1 = nf;

@@ -399,6 +399,7 @@ static int load_impl(cdlgb_ctx* c, const float* onehot, const uint8_t* codes, in
     ST_TRY(dev_alloc(c, (void**)&c->S, n * 4));
     int st = admm_alloc(c);
     if (st == CDLGB_OK && c->fused) st = fused_setup(c);
+    if (st == CDLGB_OK) c->xconv = xconv_plan_create(c, c->fused ? fused_multi_slots(c) : 0, &st);
     if (st != CDLGB_OK) {
         std::string msg = c->err;
         cudaGetLastError();

@@ -119,6 +119,8 @@ struct cdlgb_ctx {
 
     // fused path twiddles / plan
     void* fplan = nullptr;
+    // the convolution X-step (xconv.cu), taken by code updates while set
+    void* xconv = nullptr;
 
     void* plans = nullptr;          // cuFFT plan cache keyed by (direction, batch)
     int chunk = 0;                  // sequences per chunk of the cuFFT-transform passes
@@ -234,6 +236,14 @@ int warp_plan_filters(void* p);
 int fused_autotune(cdlgb_ctx* c, int maxc, double* ms, int32_t* kind, int32_t* cs, int32_t* mc,
                    int32_t* n_out, int32_t* chosen);
 int fused_has_multi(cdlgb_ctx* c);
+int fused_multi_slots(cdlgb_ctx* c);      // filter slots of the multi-iteration kernel, 0 without one
+// ---- xconv.cu (X-steps by short convolutions) ----
+void* xconv_plan_create(cdlgb_ctx* c, int slots, int* status);
+void xconv_plan_free(cdlgb_ctx* c, void* p);
+int xconv_xsteps(cdlgb_ctx* c, void* p, const float* Xin, float* Xout, int iters, int Nlim);
+int xconv_absx(void* p, const double** part, int* n);
+int xconv_plan_parts(void* p);
+int xconv_plan_filters(void* p);
 // api.cu: FASTA text -> one byte per base (the reference's parsing rules), and a load
 // from those bytes
 #include <vector>

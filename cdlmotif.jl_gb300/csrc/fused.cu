@@ -692,6 +692,11 @@ int fused_has_multi(cdlgb_ctx* c) {
     return P && P->iter;
 }
 
+int fused_multi_slots(cdlgb_ctx* c) {
+    FusedPlan* P = (FusedPlan*)c->fplan;
+    return P && P->iter ? iter_plan_cluster(P->iter) * iter_plan_filters(P->iter) : 0;
+}
+
 int fused_xsteps(cdlgb_ctx* c, const float* Xin, float* Xout, int iters) {
     FusedPlan* P = (FusedPlan*)c->fplan;
     return iter_xsteps(c, P->iter, Xin, Xout, iters);
@@ -749,7 +754,7 @@ int fused_autotune(cdlgb_ctx* c, int maxc, double* ms, int32_t* kind, int32_t* c
         for (int i = 0; i < (int)cands.size(); ++i) {
             if (i == keep) continue;
             if (cands[i].kind == 1) iter_plan_free(c, cands[i].plan);
-            else warp_plan_free(c, cands[i].plan);
+            else if (cands[i].kind == 2) warp_plan_free(c, cands[i].plan);
         }
     };
     int st = CDLGB_OK;
@@ -764,6 +769,7 @@ int fused_autotune(cdlgb_ctx* c, int maxc, double* ms, int32_t* kind, int32_t* c
         if (st != CDLGB_OK) { free_all(-1); return st; }
         if (wp) cands.push_back({2, wp});
     }
+    if (c->xconv) cands.push_back({3, c->xconv});       // the convolution X-step, where it is in use
     if (cands.empty()) return cdlgb_seterr(c, CDLGB_ENOTSUP, "autotune: no candidate");
     if ((int)cands.size() > maxc) {
         free_all(-1);
@@ -802,6 +808,7 @@ int fused_autotune(cdlgb_ctx* c, int maxc, double* ms, int32_t* kind, int32_t* c
     };
     auto run = [&](const Cand& k, int iters) -> int {
         if (k.kind == 1) return iter_xsteps_n(c, k.plan, X, X, iters, Nl);
+        if (k.kind == 3) return xconv_xsteps(c, k.plan, X, X, iters, Nl);
         for (int it = 0; it < iters; ++it) ST_TRY(warp_xstep_n(c, k.plan, X, X, Nl));
         return CDLGB_OK;
     };
@@ -827,9 +834,11 @@ int fused_autotune(cdlgb_ctx* c, int maxc, double* ms, int32_t* kind, int32_t* c
         if (rc == CDLGB_OK) rc = copy(false);
         const double per = (double)t / kIters;
         ms[i] = per;
-        kind[i] = cands[i].kind;
-        cs[i] = cands[i].kind == 1 ? iter_plan_cluster(cands[i].plan) : warp_plan_cluster(cands[i].plan);
-        mc[i] = cands[i].kind == 1 ? iter_plan_filters(cands[i].plan) : warp_plan_filters(cands[i].plan);
+        kind[i] = cands[i].kind == 2 ? 2 : 1;
+        cs[i] = cands[i].kind == 1 ? iter_plan_cluster(cands[i].plan)
+              : cands[i].kind == 2 ? warp_plan_cluster(cands[i].plan) : xconv_plan_parts(cands[i].plan);
+        mc[i] = cands[i].kind == 1 ? iter_plan_filters(cands[i].plan)
+              : cands[i].kind == 2 ? warp_plan_filters(cands[i].plan) : xconv_plan_filters(cands[i].plan);
         if (rc == CDLGB_OK && (best < 0 || per < best_ms)) { best = i; best_ms = per; }
     }
     if (e0) cudaEventDestroy(e0);
@@ -837,14 +846,20 @@ int fused_autotune(cdlgb_ctx* c, int maxc, double* ms, int32_t* kind, int32_t* c
     cudaFreeAsync(snap, s);
     if (rc != CDLGB_OK) { free_all(-1); return rc; }
     CU_TRY(c, cudaStreamSynchronize(s));
-    // keep the winner
-    iter_plan_free(c, P->iter);
-    warp_plan_free(c, P->warp);
-    P->iter = nullptr;
-    P->warp = nullptr;
-    if (cands[best].kind == 1) P->iter = cands[best].plan;
-    else P->warp = cands[best].plan;
-    free_all(best);
+    // keep the winner (the FFT form stays behind a winning convolution X-step)
+    if (cands[best].kind == 3) {
+        free_all(-1);
+    } else {
+        xconv_plan_free(c, c->xconv);
+        c->xconv = nullptr;
+        iter_plan_free(c, P->iter);
+        warp_plan_free(c, P->warp);
+        P->iter = nullptr;
+        P->warp = nullptr;
+        if (cands[best].kind == 1) P->iter = cands[best].plan;
+        else P->warp = cands[best].plan;
+        free_all(best);
+    }
     c->absx_fused = 0;           // the partial sums of |X| belong to the timing runs
     *n_out = (int32_t)cands.size();
     *chosen = best;

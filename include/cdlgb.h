@@ -221,7 +221,9 @@ int cdlgb_scan_both(cdlgb_ctx* ctx, const float* pwms, const int32_t* lens,
  * on a prefix of the loaded sequences, restoring that prefix's state after each run,
  * and keeps the fastest for the following code updates.  Per candidate i <
  * *n_candidates: ms_per_xstep[i], kind[i] (1 multi-iteration, 2 one X-step),
- * cluster[i] (CTAs per cluster), filters[i] (filters per CTA); *chosen = the winner.
+ * cluster[i] (CTAs per cluster), filters[i] (filters per CTA); *chosen = the winner.  Where
+ * the context runs the convolution X-step, that is a candidate of kind 1 as well (all
+ * iterations per call; cluster = CTAs per sequence).
  * Needs an initialised state and the fused path (CDLGB_ENOTSUP otherwise). */
 int cdlgb_autotune(cdlgb_ctx* ctx, int32_t max_candidates, double* ms_per_xstep, int32_t* kind,
                    int32_t* cluster, int32_t* filters, int32_t* n_candidates, int32_t* chosen);
