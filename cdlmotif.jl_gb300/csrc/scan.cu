@@ -8,6 +8,7 @@
 #include "cdlgb_internal.h"
 
 #include <math.h>
+#include <algorithm>
 #include <vector>
 
 namespace {
@@ -508,6 +509,250 @@ __global__ void k_scan_both_sparse16(const float* __restrict__ data, const float
     }
 }
 
+// ---------------------------------------------------------------- filtered scans
+// The best window of a motif needs the exact, ordered sum at few windows only.  Every
+// window gets an approximate score first, in steps of 1 / scale with scale * sum_i max_j
+// |pwm[j, i]| = 32000: tables of the sum over four bases, rounded to a step, both strands
+// in the halves of one integer (256 entries per four columns; the first four's entries
+// hold 32768, so a sum's halves are its strands' scores + 32768 and never carry).  Sums of
+// rounded entries add exactly, so an approximation is within half a step per segment of
+// the real sum, and the float32 sum in any order within 0.06 steps of that: eps =
+// segments / 2 + 1 steps holds.  A motif whose best approximation stays eps below its
+// threshold has no hit (nine in ten at the usual p-value); else the windows within 2 eps
+// of the best approximation are summed exactly, in the reference's order, and the first
+// maximum among them is the first maximum of all.  Sequences with a column that is not
+// one base take the exact sums for all windows.
+// Instructions bound it.  N = 20000, L = 200, K = 32: 1.24 ms for both strands with the
+// sparse sums of every window, 0.33 ms so (0.41 with half-precision tables, whose eps of
+// 0.4 % sends a third of the motifs to the exact sums); forward, N = 10000, K = 24: 0.44, 0.15.
+constexpr int kLutWarps = 16, kLutBlocks = 8;             // 32-position blocks in registers at a time
+constexpr int kLutSegs = 104;                             // KB of tables per CTA (two CTAs per SM)
+
+struct LutArgs {
+    const float* data;
+    const float* pwms;      // (K, 4, maxlen) col-major
+    const int32_t* lens;
+    const float* thresh;
+    const int32_t* limit;   // [K] best approximations (+ 32768) from here on may hit
+    const float* scale;
+    int32_t* pos;
+    float* score;
+    uint8_t* comp;
+    int K, KG, maxlen, L, N, words;                       // words: 32-position words of a sequence
+};
+
+// the larger of each 16-bit half
+__device__ __forceinline__ unsigned max_halves(unsigned a, unsigned b) {
+    unsigned r;
+    asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+
+// the window's exact sums (order of k_scan_both / k_scan_fwd), m: the masks of its bases,
+// p: the motif, [column][base]
+template <bool BOTH>
+__device__ __forceinline__ float2 exact_sums(const float* __restrict__ p, int w, const unsigned (&m)[4]) {
+    float2 s = make_float2(0.f, 0.f);
+    if (BOTH) {
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j) {
+            unsigned b = j == 0 ? m[0] : j == 1 ? m[1] : j == 2 ? m[2] : m[3];
+            for (; b; b &= b - 1) {
+                const int i = __ffs((int)b) - 1;
+                s.x = __fadd_rn(s.x, p[4 * i + j]);
+                s.y = __fadd_rn(s.y, p[4 * (w - 1 - i) + 3 - j]);
+            }
+        }
+    } else {
+#pragma unroll 1
+        for (int i = 0; i < w; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (m[j] >> i & 1) s.x = __fadd_rn(s.x, p[4 * i + j]);
+    }
+    return s;
+}
+
+template <bool BOTH>
+__global__ void __launch_bounds__(32 * kLutWarps, 2) k_scan_lut(const __grid_constant__ LutArgs A) {
+    extern __shared__ unsigned lut[];
+    const int L = A.L, K = A.K, words = A.words;
+    const int k0 = blockIdx.y * A.KG, k1 = min(K, k0 + A.KG);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned full = 0xffffffffu;
+    // the motifs, [motif][column][base], behind the tables and the warps' planes
+    const int kl = 4 * A.maxlen;
+    int segs = 0;
+    for (int k = k0; k < k1; ++k) segs += (A.lens[k] + 3) / 4;
+    unsigned* planes = reinterpret_cast<unsigned*>(lut + 256 * segs) + warp * 4 * (words + 1);   // [4][words + 1]
+    float* pw = reinterpret_cast<float*>(reinterpret_cast<unsigned*>(lut + 256 * segs) + kLutWarps * 4 * (words + 1));
+    for (int e = threadIdx.x; e < (k1 - k0) * kl; e += blockDim.x) {
+        const int k = e % (k1 - k0), r = e / (k1 - k0);               // pwms: motif fastest
+        pw[k * kl + r] = A.pwms[k0 + k + (size_t)K * r];
+    }
+    __syncthreads();
+    for (int k = k0, at = 0; k < k1; ++k) {
+        const int w = A.lens[k], ns = (w + 3) / 4;
+        const float* p = pw + (k - k0) * kl;
+        const float sc = A.scale[k];
+        for (int e = threadIdx.x; e < 256 * ns; e += blockDim.x) {
+            const int i0 = e >> 8 << 2;
+            float f = 0.f, c = 0.f;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                // base = bit q of the low nibble + 2 (bit q of the high nibble)
+                const int i = i0 + q, b = (e >> q & 1) | (e >> (4 + q) & 1) << 1;
+                if (i < w) {
+                    f += p[4 * i + b];
+                    if (BOTH) c += p[4 * (w - 1 - i) + 3 - b];
+                }
+            }
+            const int fi = __float2int_rn(f * sc) + (i0 == 0 ? 32768 : 0), ci = __float2int_rn(c * sc) + (i0 == 0 ? 32768 : 0);
+            lut[256 * at + e] = ((unsigned)ci << 16) + (unsigned)fi;
+        }
+        at += ns;
+    }
+    __syncthreads();
+    for (int n = blockIdx.x * kLutWarps + warp; n < A.N; n += gridDim.x * kLutWarps) {
+        const float* col = A.data + (size_t)n * 4 * L;
+        bool odd = false;
+        __syncwarp();
+        for (int v = 0; v <= words; ++v) {
+            const int l = 32 * v + lane;
+            const unsigned b = l < L ? base_bits(col, l) : 0u;
+            odd |= l < L && (b == 0 || (b & (b - 1)) != 0);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const unsigned m = __ballot_sync(full, b >> j & 1);
+                if (lane == j) planes[j * (words + 1) + v] = m;
+            }
+        }
+        odd = __any_sync(full, odd);
+        __syncwarp();
+        // the masks of the 32 bases from this lane's position in word v on
+        const auto masks = [&](int v, unsigned (&m)[4]) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const unsigned* pl = planes + j * (words + 1) + v;
+                m[j] = __funnelshift_r(pl[0], pl[1], lane);
+            }
+        };
+        // table indices of the windows' eight segments, a byte each
+        uint2 win[kLutBlocks];
+        const auto windows = [&](int v0) {
+#pragma unroll
+            for (int u = 0; u < kLutBlocks; ++u) {
+                win[u] = make_uint2(0u, 0u);
+                if (v0 + u < words) {
+                    unsigned m[4];
+                    masks(v0 + u, m);
+                    const unsigned lo = m[1] | m[3], hi = m[2] | m[3];
+                    const auto nibbles = [](unsigned x) {             // 16 bits -> a nibble per byte
+                        x = (x | x << 8) & 0x00ff00ffu;
+                        return (x | x << 4) & 0x0f0f0f0fu;
+                    };
+                    win[u].x = nibbles(lo & 0xffffu) | nibbles(hi & 0xffffu) << 4;
+                    win[u].y = nibbles(lo >> 16) | nibbles(hi >> 16) << 4;
+                }
+            }
+        };
+        const int groups = (words + kLutBlocks - 1) / kLutBlocks;
+        if (groups == 1) windows(0);
+        int rp = 0;
+        float rs = 0.f;
+        unsigned rc = 0;
+        const unsigned* tab = lut;
+        for (int k = k0; k < k1; ++k) {
+            const int w = A.lens[k], ns = (w + 3) / 4, eps = ns / 2 + 1, limit = A.limit[k];
+            const float thr = A.thresh[k];
+            unsigned acc[kLutBlocks];
+            const auto approximate = [&](int v0) {
+#pragma unroll
+                for (int u = 0; u < kLutBlocks; ++u) acc[u] = 0u;
+#pragma unroll
+                for (int sg = 0; sg < 8; ++sg) {
+                    if (sg >= ns) break;
+                    const unsigned* t = tab + 256 * sg;
+#pragma unroll
+                    for (int u = 0; u < kLutBlocks; ++u)
+                        if (v0 + u < words)
+                            acc[u] += t[__byte_perm(sg < 4 ? win[u].x : win[u].y, 0u, 0x4440u + (sg & 3))];
+                }
+                // windows that leave the sequence are below every other (whose halves are >= 768)
+#pragma unroll
+                for (int u = 0; u < kLutBlocks; ++u)
+                    if (32 * (v0 + u) + lane > L - w) acc[u] = 0u;
+            };
+            unsigned best = 0u;
+            for (int g = 0; g < groups; ++g) {
+                if (groups > 1) windows(kLutBlocks * g);
+                approximate(kLutBlocks * g);
+#pragma unroll
+                for (int u = 0; u < kLutBlocks; ++u) best = max_halves(best, acc[u]);
+            }
+            tab += 256 * ns;
+            int mf = (int)(best & 0xffffu), mc = BOTH ? (int)(best >> 16) : 0;
+            VI bf{-INFINITY, 0x7fffffff}, bc{-INFINITY, 0x7fffffff};
+            if (odd || __any_sync(full, max(mf, mc) >= limit)) {
+                mf = __reduce_max_sync(full, mf);
+                mc = __reduce_max_sync(full, mc);
+                // a strand that is 2 eps behind cannot win
+                const int cf = mf >= mc - 2 * eps ? mf - 2 * eps : 0x10000;
+                const int cc = BOTH && mc >= mf - 2 * eps ? mc - 2 * eps : 0x10000;
+                for (int g = 0; g < groups; ++g) {
+                    if (groups > 1) {
+                        tab -= 256 * ns;
+                        windows(kLutBlocks * g);
+                        approximate(kLutBlocks * g);
+                        tab += 256 * ns;
+                    }
+#pragma unroll
+                    for (int u = 0; u < kLutBlocks; ++u) {
+                        const int v = kLutBlocks * g + u, l = 32 * v + lane;
+                        const bool cand = v < words && l <= L - w &&
+                                          (odd || (int)(acc[u] & 0xffffu) >= cf || (BOTH && (int)(acc[u] >> 16) >= cc));
+                        if (!cand) continue;
+                        unsigned m[4];
+                        masks(v, m);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) m[j] &= w == 32 ? full : (1u << w) - 1u;
+                        const float2 s = exact_sums<BOTH>(pw + (k - k0) * kl, w, m);
+                        if (s.x > bf.v) bf = VI{s.x, l};
+                        if (BOTH && s.y > bc.v) bc = VI{s.y, l};
+                    }
+                }
+                for (int o = 16; o > 0; o >>= 1) {
+                    VI y;
+                    y.v = __shfl_xor_sync(full, bf.v, o);
+                    y.i = __shfl_xor_sync(full, bf.i, o);
+                    bf = vi_best(bf, y);
+                    if (BOTH) {
+                        y.v = __shfl_xor_sync(full, bc.v, o);
+                        y.i = __shfl_xor_sync(full, bc.i, o);
+                        bc = vi_best(bc, y);
+                    }
+                }
+            }
+            const bool fwd = bf.v >= bc.v;                // forward kept on ties
+            const VI b = fwd ? bf : bc;
+            const bool hit = b.v > thr;
+            const int at = (k - k0) & 31;
+            if (lane == at) {
+                // REF_QUIRK_Q3: the forward scan's best hit at the first position reads as none
+                rp = hit && (BOTH || b.i != 0) ? b.i + 1 : 0;
+                rs = hit ? b.v : 0.f;
+                rc = hit && !fwd;
+            }
+            if ((at == 31 || k == k1 - 1) && lane <= at) {
+                const size_t o = (k - at + lane) + (size_t)K * n;
+                if (A.pos) A.pos[o] = rp;
+                if (BOTH && A.score) A.score[o] = rs;
+                if (BOTH && A.comp) A.comp[o] = (uint8_t)rc;
+            }
+        }
+    }
+}
+
 // the sparse scans apply: exact 0/1 data, finite PWM entries (within each motif's
 // length), not turned off by CDLGB_SCAN_DENSE
 bool sparse_ok(const cdlgb_ctx* c, const float* pwms, const int32_t* lens, int K, int maxlen) {
@@ -564,17 +809,71 @@ int check_pwm_args(cdlgb_ctx* c, const float* pwms, const int32_t* lens, const f
     return CDLGB_OK;
 }
 
+// The filtered scans take motifs of at most 32 columns and sequences of at most 4096 bases;
+// the forward scan's threshold is not negative (below zero its first maximum can be a
+// window that is no hit).  Fills the motifs' scales and limits (as floats' bits) and the
+// motifs per CTA.
+bool lut_ok(const cdlgb_ctx* c, const float* pwms, const int32_t* lens, const float* thresh, int K, int maxlen,
+            bool both, std::vector<float>& meta, int* KG) {
+    if (maxlen > 32 || c->L4 / 4 > 4096 || !sparse_ok(c, pwms, lens, K, maxlen)) return false;
+    meta.resize(2 * (size_t)K);
+    int segs = 0, most = 1;
+    for (int k = 0; k < K; ++k) {
+        if (!both && !(thresh[k] >= 0.f)) return false;
+        double S = 0.0;
+        for (int i = 0; i < lens[k]; ++i) {
+            float a = 0.f;
+            for (int j = 0; j < 4; ++j) a = fmaxf(a, fabsf(pwms[k + (size_t)K * (j + 4 * i)]));
+            S += a;
+        }
+        // sums in float32 have to stay far from its range's ends
+        if (!(S < 1e30) || (S > 0.0 && S < 1e-25)) return false;
+        const int ns = (lens[k] + 3) / 4;
+        const float scale = S > 0.0 ? (float)(32000.0 / S) : 0.f;
+        meta[k] = scale;
+        const double at = floor((double)scale * (double)thresh[k]) + 32768.0 - (ns / 2 + 1);
+        // a NaN threshold has no hit; a motif of zeros is left to the exact sums
+        const int32_t limit = thresh[k] != thresh[k] ? 65536 : scale == 0.f ? 1
+                            : at > 65536.0 ? 65536 : at < 1.0 ? 1 : (int32_t)at;
+        memcpy(&meta[K + k], &limit, 4);
+        segs += ns;
+        most = ns > most ? ns : most;
+    }
+    const int parts = (segs + kLutSegs - 1) / kLutSegs;
+    *KG = std::min((K + parts - 1) / parts, kLutSegs / most);
+    return true;
+}
+
 // device scratch layout: [pwms K*4*maxlen f32][thresh K f32] and [lens K i32][pos K*N i32]
 int upload_pwms(cdlgb_ctx* c, const float* pwms, const int32_t* lens, const float* thresh, int K,
                 int maxlen, size_t extra_i) {
     size_t nf = (size_t)K * 4 * maxlen + K;
-    ST_TRY(ensure_scratch(c, &c->scan_f, &c->scan_f_cap, nf + (size_t)K * c->N));
+    ST_TRY(ensure_scratch(c, &c->scan_f, &c->scan_f_cap, nf + (size_t)K * c->N + 2 * (size_t)K));
     ST_TRY(ensure_scratch(c, &c->scan_i, &c->scan_i_cap, (size_t)K + extra_i));
     CU_TRY(c, cudaMemcpyAsync(c->scan_f, pwms, (size_t)K * 4 * maxlen * 4, cudaMemcpyHostToDevice,
                               c->stream));
     CU_TRY(c, cudaMemcpyAsync(c->scan_f + (size_t)K * 4 * maxlen, thresh, (size_t)K * 4,
                               cudaMemcpyHostToDevice, c->stream));
     CU_TRY(c, cudaMemcpyAsync(c->scan_i, lens, (size_t)K * 4, cudaMemcpyHostToDevice, c->stream));
+    return CDLGB_OK;
+}
+
+// the filtered scan of one or both strands; dmeta: 2 K floats of device scratch
+template <bool BOTH>
+int launch_lut(cdlgb_ctx* c, const std::vector<float>& meta, int KG, int K, int maxlen, int32_t* dpos, float* dscore,
+               uint8_t* dcomp, float* dmeta) {
+    CU_TRY(c, cudaMemcpyAsync(dmeta, meta.data(), (size_t)K * 8, cudaMemcpyHostToDevice, c->stream));
+    LutArgs a;
+    a.data = scan_data(c); a.pwms = c->scan_f; a.lens = c->scan_i; a.thresh = c->scan_f + (size_t)K * 4 * maxlen;
+    a.scale = dmeta; a.limit = reinterpret_cast<const int32_t*>(dmeta + K); a.pos = dpos; a.score = dscore; a.comp = dcomp;
+    a.K = K; a.KG = KG; a.maxlen = maxlen; a.L = c->L4 / 4; a.N = c->N; a.words = (a.L + 31) / 32;
+    const size_t shm = (size_t)KG * ((maxlen + 3) / 4) * 1024 + (size_t)kLutWarps * 16 * (a.words + 1) +
+                       (size_t)KG * 16 * maxlen;
+    CU_TRY(c, cudaFuncSetAttribute(k_scan_lut<BOTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 150 * 1024));
+    const int parts = (K + KG - 1) / KG;
+    const int gx = std::max(1, std::min((c->N + kLutWarps - 1) / kLutWarps, 2 * 152 / parts));
+    k_scan_lut<BOTH><<<dim3(gx, parts), 32 * kLutWarps, shm, c->stream>>>(a);
+    LAUNCH_CHECK(c, "k_scan_lut");
     return CDLGB_OK;
 }
 
@@ -594,7 +893,12 @@ int scan_fwd(cdlgb_ctx* c, const float* pwms, const int32_t* lens, const float* 
     const int nts = ((L + 31) / 32) * 32;
     const size_t shs = (size_t)K * 4 * maxlen * sizeof(float) + (size_t)K * (nts / 32) * sizeof(VI) +
                        (size_t)L;
-    if (nts <= 1024 && shs <= 64 * 1024 && sparse_ok(c, pwms, lens, K, maxlen)) {
+    std::vector<float> meta;
+    int KG = 0;
+    if (lut_ok(c, pwms, lens, thresh, K, maxlen, false, meta, &KG)) {
+        ST_TRY(launch_lut<false>(c, meta, KG, K, maxlen, dpos, nullptr, nullptr,
+                                 c->scan_f + (size_t)K * 4 * maxlen + K + (size_t)K * N));
+    } else if (nts <= 1024 && shs <= 64 * 1024 && sparse_ok(c, pwms, lens, K, maxlen)) {
         if (shs > 48 * 1024)
             CU_TRY(c, cudaFuncSetAttribute(k_scan_fwd_sparse, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            64 * 1024));
@@ -636,7 +940,11 @@ int scan_both(cdlgb_ctx* c, const float* pwms, const int32_t* lens, const float*
                        (size_t)4 * ((L + 31) / 32 + 2) * sizeof(uint32_t);
     const size_t shq = (size_t)K * 64 * sizeof(float2) + (size_t)K * (nts / 32) * 2 * sizeof(VI) +
                        (size_t)4 * ((L + 31) / 32 + 2) * sizeof(uint32_t);
-    if (nts <= 1024 && maxlen <= 16 && shq <= 64 * 1024 && sparse_ok(c, pwms, lens, K, maxlen)) {
+    std::vector<float> meta;
+    int KG = 0;
+    if (lut_ok(c, pwms, lens, thresh, K, maxlen, true, meta, &KG)) {
+        ST_TRY(launch_lut<true>(c, meta, KG, K, maxlen, dpos, dscore, c->scan_u, dscore + (size_t)K * N));
+    } else if (nts <= 1024 && maxlen <= 16 && shq <= 64 * 1024 && sparse_ok(c, pwms, lens, K, maxlen)) {
         if (shq > 48 * 1024)
             CU_TRY(c, cudaFuncSetAttribute(k_scan_both_sparse16, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            64 * 1024));
