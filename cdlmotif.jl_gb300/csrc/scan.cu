@@ -1116,61 +1116,89 @@ namespace {
 // reached keys in ascending order.
 constexpr int kTouzetMaxR = 6144;     // score range per PWM (two uint64 tables in smem)
 
-__global__ void k_touzet(const int32_t* __restrict__ kq, const int32_t* __restrict__ lens,
-                         const int32_t* __restrict__ kmin, const int32_t* __restrict__ range,
-                         int maxlen, const unsigned long long* __restrict__ thr_count,
-                         int32_t* __restrict__ alpha_k, int32_t* __restrict__ status) {
+// The table's last pass (tail sums) runs in parallel: one thread over up to 6144 entries
+// twice was 55 of the kernel's 74 us at widths of 20 columns.
+constexpr int kTouzetThreads = 256;
+__global__ void __launch_bounds__(kTouzetThreads) k_touzet(
+    const int32_t* __restrict__ kq, const int32_t* __restrict__ lens, const int32_t* __restrict__ kmin,
+    const int32_t* __restrict__ range, int maxlen, const unsigned long long* __restrict__ thr_count,
+    int32_t* __restrict__ alpha_k, int32_t* __restrict__ status) {
     extern __shared__ unsigned long long tab[];
+    __shared__ unsigned long long part[kTouzetThreads];
+    __shared__ int first[kTouzetThreads / 32], last[kTouzetThreads / 32];
     const int p = blockIdx.x;
     const int m = lens[p], R = range[p];
     unsigned long long* Q0 = tab;
     unsigned long long* Q1 = tab + kTouzetMaxR;
     const int32_t* kp = kq + (size_t)p * 4 * maxlen;       // k[j][i] at j * maxlen + i
-    for (int s = threadIdx.x; s < R; s += blockDim.x) Q0[s] = 0ull;
-    __syncthreads();
     if (threadIdx.x == 0) Q0[0] = 1ull;
     __syncthreads();
     int lo = 0;      // sum of the column minima so far
     int width = 1;   // reached keys lie in [lo, lo + width)
     for (int i = 0; i < m; ++i) {
-        int cmin = kp[i], cmax = kp[i];
-        for (int j = 1; j < 4; ++j) {
-            cmin = min(cmin, kp[j * maxlen + i]);
-            cmax = max(cmax, kp[j * maxlen + i]);
-        }
+        int k[4];
+        for (int j = 0; j < 4; ++j) k[j] = kp[j * maxlen + i];
+        const int cmin = min(min(k[0], k[1]), min(k[2], k[3])), cmax = max(max(k[0], k[1]), max(k[2], k[3]));
         const int nw = width + (cmax - cmin);
-        for (int s = threadIdx.x; s < nw; s += blockDim.x) {
+        for (int s = threadIdx.x; s < nw; s += kTouzetThreads) {
             unsigned long long acc = 0ull;
             for (int j = 0; j < 4; ++j) {
-                const int src = s - (kp[j * maxlen + i] - cmin);
+                const int src = s - (k[j] - cmin);
                 if (src >= 0 && src < width) acc += Q0[src];
             }
             Q1[s] = acc;
         }
         __syncthreads();
-        for (int s = threadIdx.x; s < nw; s += blockDim.x) Q0[s] = Q1[s];
-        __syncthreads();
+        unsigned long long* t = Q0;
+        Q0 = Q1;
+        Q1 = t;
         lo += cmin;
         width = nw;
     }
+    if (lo != kmin[p] || width != R) {
+        if (threadIdx.x == 0) status[p] = 1;
+        return;
+    }
+    // find_largest_alpha: q_sum starts at the total (4^m counts), keys ascending;
+    // q_sum >= pval  <=>  tail >= ceil(pval 4^m)  (integers, exact).  The answer is the first
+    // reached key whose tail is below, or the last reached key.  Thread t takes keys
+    // [t per, (t + 1) per); tails of whole threads' keys by a suffix sum over the threads.
+    const int per = (width + kTouzetThreads - 1) / kTouzetThreads;
+    const int s0 = threadIdx.x * per, s1 = min(width, s0 + per);
+    unsigned long long sum = 0ull;
+    int end = -1;
+    for (int s = s0; s < s1; ++s) {
+        sum += Q0[s];
+        if (Q0[s]) end = s;
+    }
+    part[threadIdx.x] = sum;
+    for (int o = 1; o < kTouzetThreads; o <<= 1) {
+        __syncthreads();
+        const unsigned long long v = threadIdx.x + o < kTouzetThreads ? part[threadIdx.x + o] : 0ull;
+        __syncthreads();
+        part[threadIdx.x] += v;
+    }
+    unsigned long long tail = part[threadIdx.x];             // keys from s0 on
+    int at = 0x7fffffff;
+    for (int s = s0; s < s1 && at == 0x7fffffff; ++s) {
+        const unsigned long long v = Q0[s];
+        if (v == 0ull) continue;                             // keys never reached are absent
+        if (tail < thr_count[p]) at = s;
+        tail -= v;
+    }
+    at = __reduce_min_sync(0xffffffffu, at);
+    end = __reduce_max_sync(0xffffffffu, end);
+    if ((threadIdx.x & 31) == 0) {
+        first[threadIdx.x >> 5] = at;
+        last[threadIdx.x >> 5] = end;
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
-        if (lo != kmin[p] || width != R) {
-            status[p] = 1;
-            return;
+        for (int w = 1; w < kTouzetThreads / 32; ++w) {
+            at = min(at, first[w]);
+            end = max(end, last[w]);
         }
-        // find_largest_alpha: q_sum starts at the total (4^m counts), keys ascending;
-        // q_sum >= pval  <=>  tail >= ceil(pval 4^m)  (integers, exact)
-        unsigned long long tail = 0ull;
-        for (int s = 0; s < width; ++s) tail += Q0[s];
-        int best = -1;
-        for (int s = 0; s < width; ++s) {
-            const unsigned long long v = Q0[s];
-            if (v == 0ull) continue;                       // keys never reached are absent
-            best = s;
-            if (tail < thr_count[p]) break;
-            tail -= v;
-        }
-        alpha_k[p] = lo + best;
+        alpha_k[p] = lo + (at != 0x7fffffff ? at : end);
         status[p] = 0;
     }
 }
@@ -1184,7 +1212,7 @@ int touzet_thresholds(cdlgb_ctx* c, const float* pwms, const int32_t* lens, int 
     const double eps = 1e-1;                                 // _granularity_
     const size_t nk = (size_t)K * 4 * maxlen;
     std::vector<int32_t> host((size_t)nk + 5 * (size_t)K, 0);
-    int32_t* kq = host.data();
+    int32_t* kq = host.data() + 2 * (size_t)K;
     int32_t* kmin = kq + nk;
     int32_t* range = kmin + K;
     int32_t* hl = range + K;
@@ -1221,23 +1249,20 @@ int touzet_thresholds(cdlgb_ctx* c, const float* pwms, const int32_t* lens, int 
         range[p] = (int32_t)(hi - lo + 1);
         thr[p] = (unsigned long long)ceil(ldexp(pval, 2 * m));   // pval 4^m is exact; <= 2^62
     }
-    ST_TRY(ensure_scratch(c, &c->scan_i, &c->scan_i_cap, nk + 5 * (size_t)K));
-    int32_t* d_kq = c->scan_i;
-    int32_t* d_lens = d_kq + nk + 2 * (size_t)K;
-    int32_t* d_alpha = d_lens + K;
+    // thr, kq, kmin, range and lens in one copy (thr first: 8-byte aligned), then alpha, status
+    const size_t up = 2 * (size_t)K + nk + 3 * (size_t)K;
+    memcpy(host.data(), thr.data(), (size_t)K * 8);
+    ST_TRY(ensure_scratch(c, &c->scan_i, &c->scan_i_cap, up + 2 * (size_t)K));
+    int32_t* d_kq = c->scan_i + 2 * (size_t)K;
+    int32_t* d_alpha = c->scan_i + up;
     int32_t* d_status = d_alpha + K;
-    unsigned long long* d_thr = nullptr;
-    CU_TRY(c, cudaMallocAsync((void**)&d_thr, (size_t)K * sizeof(unsigned long long), c->stream));
-    CU_TRY(c, cudaMemcpyAsync(d_kq, host.data(), (nk + 3 * (size_t)K) * 4, cudaMemcpyHostToDevice, c->stream));
-    CU_TRY(c, cudaMemcpyAsync(d_thr, thr.data(), (size_t)K * sizeof(unsigned long long), cudaMemcpyHostToDevice,
-                              c->stream));
+    CU_TRY(c, cudaMemcpyAsync(c->scan_i, host.data(), up * 4, cudaMemcpyHostToDevice, c->stream));
     const int shm = (int)(2 * (size_t)kTouzetMaxR * sizeof(unsigned long long));
     CU_TRY(c, cudaFuncSetAttribute(k_touzet, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
-    k_touzet<<<K, 256, shm, c->stream>>>(d_kq, d_lens, d_kq + nk, d_kq + nk + K, maxlen, d_thr, d_alpha,
-                                         d_status);
-    cudaError_t e = cudaGetLastError();
-    cudaFreeAsync(d_thr, c->stream);
-    if (e != cudaSuccess) return cdlgb_seterr(c, CDLGB_ECUDA, "k_touzet: %s", cudaGetErrorString(e));
+    k_touzet<<<K, kTouzetThreads, shm, c->stream>>>(d_kq, d_kq + nk + 2 * (size_t)K, d_kq + nk, d_kq + nk + K, maxlen,
+                                                    reinterpret_cast<const unsigned long long*>(c->scan_i), d_alpha,
+                                                    d_status);
+    LAUNCH_CHECK(c, "k_touzet");
     std::vector<int32_t> out(2 * (size_t)K);
     CU_TRY(c, cudaMemcpyAsync(out.data(), d_alpha, 2 * (size_t)K * 4, cudaMemcpyDeviceToHost, c->stream));
     CU_TRY(c, cudaStreamSynchronize(c->stream));
