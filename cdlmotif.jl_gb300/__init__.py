@@ -510,6 +510,18 @@ def extension(c: CDL, positions, lens, use_comp=None, bg=_BG, pseudocount=5.0,
     return pos, ln, dec, inc
 
 
+def _any_entry(pos: np.ndarray) -> np.ndarray:
+    """Per motif whether any position (N, K) is an entry (a reduction that vectorises along
+    the motifs; a boolean array and its any() take five times as long)."""
+    return pos.max(axis=0, initial=0) > 0
+
+
+def _columns(a: np.ndarray, keep: np.ndarray) -> np.ndarray:
+    """The kept motifs' columns of an array of this module's own, as a C-order array (take
+    is faster than a boolean column index, and needs no bounds checks here)."""
+    return a if keep.all() else a.take(np.flatnonzero(keep), axis=1, mode="clip")
+
+
 def extend(c: CDL, positions, lens, filter_size: int, use_comp=None, bg=_BG, pseudocount=5.0,
            perc_no_less_than=0.95, ic_extension_thresh=0.075, pseudocounts_r=0.0295,
            smoothing=True, re_evaluate_pfm=True) -> dict:
@@ -520,11 +532,10 @@ def extend(c: CDL, positions, lens, filter_size: int, use_comp=None, bg=_BG, pse
     "pfms" (list or None), "keep" (bool (K,))}."""
     pos, ln, _, _ = extension(c, positions, lens, use_comp, bg, pseudocount, perc_no_less_than,
                               ic_extension_thresh)
-    keep = (pos > 0).any(axis=0) & (ln > filter_size + 2)
-    kept = np.flatnonzero(keep)
-    pos = pos.take(kept, axis=1)          # (a C-order copy; faster than a boolean column index)
+    keep = _any_entry(pos) & (ln > filter_size + 2)
+    pos = _columns(pos, keep)
     ln = ln[keep]
-    uc = None if use_comp is None else np.asarray(use_comp).take(kept, axis=1)
+    uc = None if use_comp is None else _columns(np.array(use_comp), keep)
     pfms = None
     if re_evaluate_pfm:
         pfms = posdicts2pfms(c, pos, ln, uc, pseudocounts_r, pseudocount, smoothing) if len(ln) else []
@@ -576,20 +587,21 @@ def masked_trim(pfms, filter_size: int, positions=None, use_comp=None, bg=_BG,
     if positions is not None:
         # every entry (position > 0) moves by its motif's front trim, or by its back
         # trim when reverse-complemented after merging (trim.jl:47-59)
-        pos = np.array(positions, np.int32, copy=True)
+        old = np.asarray(positions, np.int32)
         if after_merged and use_comp is not None:
             shift = np.where(np.asarray(use_comp) != 0, back[None, :], front[None, :]).astype(np.int32)
         else:
             shift = front[None, :]
-        pos += (pos > 0).astype(np.int32) * shift
+        pos = np.clip(old, 0, 1)
+        pos *= shift
+        pos += old
     keep = np.array([p.shape[1] > filter_size + 1 for p in new], bool)
     if pos is not None:
-        keep &= (pos > 0).any(axis=0)
+        keep &= _any_entry(pos)
     new = [p for p, kk in zip(new, keep) if kk]
     lens = np.array([p.shape[1] for p in new], np.int32)
     out = {"pfms": new, "lens": lens, "keep": keep, "front": front, "back": back,
-           "positions": (pos.take(np.flatnonzero(keep), axis=1) if (pos is not None and update_positions)
-                         else None),
+           "positions": _columns(pos, keep) if (pos is not None and update_positions) else None,
            "use_comp": use_comp, "pwms": None, "thresh": None}
     if c is not None and len(new):
         pwms = [pfm2pwm(p, bg) for p in new]
@@ -648,8 +660,8 @@ def filter_using_evalue(c: CDL, pwms, thresh, positions, lens=None, cpu=False, n
             bg_pos, bg_sc, _ = overlapping_scan(c, pwms, thresh, ln)
             if non_overlap:
                 bg_pos, _, _ = non_overlap_scan(c, bg_pos, bg_sc, ln, None)
-    hits = (np.asarray(positions) > 0).sum(axis=0).astype(np.int32)
-    hits_bg = (bg_pos > 0).sum(axis=0).astype(np.int32)
+    hits = np.clip(positions, 0, 1).sum(axis=0, dtype=np.int32)
+    hits_bg = np.clip(bg_pos, 0, 1).sum(axis=0, dtype=np.int32)
     ev = fisher_evalues(hits, hits_bg, c.N)
     if get_evalues_only:
         return ev

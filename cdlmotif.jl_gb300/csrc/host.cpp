@@ -217,19 +217,32 @@ int cdlgb_fisher_evalues(const int32_t* hits, const int32_t* hits_bg, int32_t K,
         // c1 = a + b draws), observed a; P(X = j) = C(r1, j) C(r2, c1 - j) / C(r1 + r2, c1)
         const double r1 = (double)(a + N), r2 = (double)(b + N), c1 = (double)(a + b);
         const long lo = (long)std::max(0.0, c1 - r2), hi = (long)std::min(c1, r1);
-        auto lp = [&](long j) {
-            return -lgamma((double)j + 1.0) - lgamma(r1 - (double)j + 1.0) -
-                   lgamma(c1 - (double)j + 1.0) - lgamma(r2 - c1 + (double)j + 1.0);
+        // The probabilities relative to the largest one, from it outwards: the ratio of
+        // neighbours is rational, and falls away from the mode, so a tail's rest is below a
+        // geometric series and each sum ends once that no longer counts.
+        auto up = [&](long j) {       // P(j + 1) / P(j)
+            return ((r1 - (double)j) * (c1 - (double)j)) / (((double)j + 1.0) * (r2 - c1 + (double)j + 1.0));
         };
-        double mx = -INFINITY;
-        for (long j = lo; j <= hi; ++j) mx = std::max(mx, lp(j));
-        double left = 0.0, right = 0.0, total = 0.0;
-        for (long j = lo; j <= hi; ++j) {
-            const double t = exp(lp(j) - mx);
-            total += t;
-            if (j <= a) left += t;
-            if (j >= a) right += t;
-        }
+        auto rest = [](double t, double ratio) { return ratio < 1.0 ? t * ratio / (1.0 - ratio) : INFINITY; };
+        const long mode = std::min(hi, std::max(lo, (long)floor((r1 + 1.0) * (c1 + 1.0) / (r1 + r2 + 2.0))));
+        // sum of P(j), j = from, from + step, ... to the end, with P(from) = t
+        auto tail = [&](long from, int step, double t) {
+            double s = t;
+            for (long j = from; step > 0 ? j < hi : j > lo; j += step) {
+                const double r = step > 0 ? up(j) : 1.0 / up(j - 1);
+                if (rest(t, r) < 1e-17 * s) break;
+                s += t *= r;
+            }
+            return s;
+        };
+        double ta = 1.0;              // P(a) / P(mode); 0 once it underflows
+        for (long j = mode; j < a && ta > 0.0; ++j) ta *= up(j);
+        for (long j = mode; j > a && ta > 0.0; --j) ta /= up(j - 1);
+        const double total = tail(mode, -1, 1.0) + tail(mode, 1, 1.0) - 1.0;
+        // the side of a away from the mode is a tail; the other one is the rest
+        const double below = a <= mode ? tail(a, -1, ta) : total - tail(a, 1, ta) + ta;
+        const double above = a >= mode ? tail(a, 1, ta) : total - below + ta;
+        const double left = below, right = above;
         double p = 2.0 * std::min(left, right) / total;
         if (p > 1.0) p = 1.0;
         evalues_out[i] = p * (double)K;
