@@ -25,6 +25,7 @@
 namespace {
 
 constexpr int kBlock = 256;
+constexpr int kInitParts = 152 * 8;     // where init_x's sums of |X| begin in dred
 
 __host__ __device__ inline uint64_t splitmix64(uint64_t x) {
     x += 0x9E3779B97F4A7C15ull;
@@ -46,19 +47,6 @@ __global__ void k_bcast_plane(float4* __restrict__ dst, const float4* __restrict
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n4;
          i += (size_t)gridDim.x * blockDim.x)
         dst[i] = plane[i % pl4];
-}
-
-// DXh[n,f] = scale * sum_m Gh[m,f] Xh[n,m,f]
-__global__ void k_spec_dot(const float2* __restrict__ Xh, const float2* __restrict__ Gh,
-                           float2* __restrict__ out, int F, int M, int N, float scale) {
-    size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (t >= (size_t)F * N) return;
-    int f = (int)(t % F);
-    size_t n = t / F;
-    float2 acc = make_float2(0.f, 0.f);
-    const float2* x = Xh + n * M * F + f;
-    for (int m = 0; m < M; ++m) acc = cfma(Gh[(size_t)m * F + f], x[(size_t)m * F], acc);
-    out[t] = make_float2(acc.x * scale, acc.y * scale);
 }
 
 // A[f] = sum_m |Gh[m,f]|^2
@@ -402,38 +390,6 @@ __global__ void k_abssum(const float4* __restrict__ X, size_t n4, double* __rest
     if (threadIdx.x == 0) out[blockIdx.x] = acc;
 }
 
-// The initial X in one pass (CDL_setup.jl:191-192): standard normal on the rows
-// (l-1) % 4 == 0 and zero elsewhere.  Lg % 4 == 0, so those rows are the .x components
-// of the float4s; element 4 j draws from counter 4 j of the seed's splitmix64 stream
-// (Box-Muller on two 24-bit uniforms).  A given X0 is masked to the same rows instead.
-// Also y2 = y3 = 0 (CDL_setup.jl:220-230) and the per-block sums of |X| for the initial
-// objective.  Launched on k_abssum's grid (304 blocks of kBlock), so every thread visits
-// k_abssum's indices in its order: the same sums, bit for bit.
-__global__ void k_init_x(float4* __restrict__ X, float4* __restrict__ y2, float4* __restrict__ y3,
-                         size_t n4, uint64_t seed, int draw, double* __restrict__ out) {
-    __shared__ double sh[32];
-    double acc = 0.0;
-    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < n4;
-         j += (size_t)gridDim.x * blockDim.x) {
-        float4 v;
-        if (draw) {
-            const uint64_t h = splitmix64(seed * 0x2545F4914F6CDD1Dull ^ (uint64_t)(4 * j));
-            const float u1 = ((float)(h >> 40) + 0.5f) * (1.0f / 16777216.0f);
-            const float u2 = ((float)(h & 0xFFFFFFull) + 0.5f) * (1.0f / 16777216.0f);
-            v = make_float4(sqrtf(-2.f * logf(u1)) * cospif(2.f * u2), 0.f, 0.f, 0.f);
-        } else {
-            v = make_float4(X[j].x, 0.f, 0.f, 0.f);
-        }
-        X[j] = v;
-        y2[j] = z;
-        y3[j] = z;
-        acc += (double)((fabsf(v.x) + fabsf(v.y)) + (fabsf(v.z) + fabsf(v.w)));
-    }
-    acc = block_sum_d(acc, sh);
-    if (threadIdx.x == 0) out[blockIdx.x] = acc;
-}
-
 // Sums of many float32 terms.  A float64 sum per term is what bounds such a pass here (two
 // FP64 operations per SM and cycle: 13.2 ms for the threshold's two passes over 1.19e9
 // codes, 0.72 TB/s), so runs of 16 or 32 terms go into a compensated float32 pair first
@@ -597,13 +553,6 @@ __global__ void k_pos_final(const double* __restrict__ part, int nb, double* __r
 }
 
 // host-side seeded normal (used for D0 when none is given)
-double host_normal(uint64_t seed, uint64_t i) {
-    uint64_t h = splitmix64(seed * 0x2545F4914F6CDD1Dull ^ (i + 0x9E37ull));
-    double u1 = ((double)(h >> 11) + 0.5) * (1.0 / 9007199254740992.0);
-    uint64_t h2 = splitmix64(h);
-    double u2 = ((double)(h2 >> 11) + 0.5) * (1.0 / 9007199254740992.0);
-    return sqrt(-2.0 * log(u1)) * cos(2.0 * M_PI * u2);
-}
 double host_uniform(uint64_t seed, uint64_t i) {
     uint64_t h = splitmix64(seed * 0x9E3779B97F4A7C15ull ^ (i + 0x51ull));
     return ((double)(h >> 11) + 0.5) * (1.0 / 9007199254740992.0);
@@ -911,47 +860,41 @@ int admm_init(cdlgb_ctx* c, const float* X0, const float* D0, uint64_t seed) {
     c->outer_done = 0;
     CU_TRY(c, cudaMemsetAsync(c->dres, 0, RESIDUAL_COUNT * sizeof(double), c->stream));
     float* X = c->Xb[0];
-    // X0 (CDL_setup.jl:191-192): given, or standard normal; masked to the 4-stride; with
-    // y2 = y3 = 0 and sum |X| for the initial objective in the same pass
-    if (X0) CU_TRY(c, cudaMemcpyAsync(X, X0, LMN * 4, cudaMemcpyHostToDevice, s));
-    k_init_x<<<152 * 2, kBlock, 0, s>>>((float4*)X, (float4*)c->y2, (float4*)c->y3, LMN / 4, seed,
-                                        X0 ? 0 : 1, c->dred);
-    LAUNCH_CHECK(c, "k_init_x");
     // the spectral D-step (dspec.cu) where its transforms cover Lg and M
     c->dspec = 0;
     c->time_stale = 0;
     c->time_init = 0;
     if (c->g1h) c->dspec = 1;                 // spectral_state() held at allocation
     // D0 (CDL_setup.jl:182-183), masked by P_D
-    std::vector<float> D(LM, 0.f);
-    if (D0) {
-        for (int m = 0; m < M; ++m)
-            for (int l = 0; l < flen; ++l) D[(size_t)m * Lg + l] = D0[(size_t)m * Lg + l];
-    } else if (c->p.init_mode == 1) {
-        // the reference's draw: per 4-row group a uniform point on the simplex
-        uint64_t ctr = 0;
-        for (int m = 0; m < M; ++m)
-            for (int g = 0; g < flen / 4; ++g) {
-                double u[3];
-                for (int k = 0; k < 3; ++k) u[k] = host_uniform(seed, ctr++);
-                std::sort(u, u + 3);
-                double w[5] = {0, u[0], u[1], u[2], 1};
-                for (int k = 0; k < 4; ++k) D[(size_t)m * Lg + 4 * g + k] = (float)(w[k + 1] - w[k]);
-            }
+    if (!D0 && c->p.init_mode != 1) {
+        ST_TRY(init_d(c, seed));
     } else {
-        uint64_t ctr = 0;
-        for (int m = 0; m < M; ++m) {
-            double nrm = 0;
-            std::vector<double> v(flen);
-            for (int l = 0; l < flen; ++l) { v[l] = host_normal(seed, ctr++); nrm += v[l] * v[l]; }
-            nrm = sqrt(nrm);
-            for (int l = 0; l < flen; ++l) D[(size_t)m * Lg + l] = (float)(v[l] / nrm);
+        std::vector<float> D(LM, 0.f);
+        if (D0) {
+            for (int m = 0; m < M; ++m)
+                for (int l = 0; l < flen; ++l) D[(size_t)m * Lg + l] = D0[(size_t)m * Lg + l];
+        } else {
+            // the reference's draw: per 4-row group a uniform point on the simplex
+            uint64_t ctr = 0;
+            for (int m = 0; m < M; ++m)
+                for (int g = 0; g < flen / 4; ++g) {
+                    double u[3];
+                    for (int k = 0; k < 3; ++k) u[k] = host_uniform(seed, ctr++);
+                    std::sort(u, u + 3);
+                    double w[5] = {0, u[0], u[1], u[2], 1};
+                    for (int k = 0; k < 4; ++k) D[(size_t)m * Lg + 4 * g + k] = (float)(w[k + 1] - w[k]);
+                }
         }
+        CU_TRY(c, cudaMemcpyAsync(c->G1, D.data(), LM * 4, cudaMemcpyHostToDevice, s));
+        CU_TRY(c, cudaMemcpyAsync(c->G3, c->G1, LM * 4, cudaMemcpyDeviceToDevice, s));
+        CU_TRY(c, cudaMemcpyAsync(c->Dbest, c->G1, LM * 4, cudaMemcpyDeviceToDevice, s));
+        CU_TRY(c, cudaMemcpyAsync(c->dsum, c->G1, LM * 4, cudaMemcpyDeviceToDevice, s));
     }
-    CU_TRY(c, cudaMemcpyAsync(c->G1, D.data(), LM * 4, cudaMemcpyHostToDevice, s));
-    CU_TRY(c, cudaMemcpyAsync(c->G3, c->G1, LM * 4, cudaMemcpyDeviceToDevice, s));
-    CU_TRY(c, cudaMemcpyAsync(c->Dbest, c->G1, LM * 4, cudaMemcpyDeviceToDevice, s));
-    CU_TRY(c, cudaMemcpyAsync(c->dsum, c->G1, LM * 4, cudaMemcpyDeviceToDevice, s));
+    // X0 (CDL_setup.jl:191-192): given, or standard normal; masked to the 4-stride; with
+    // y2 = y3 = 0, DX = real(ifft(sum_m D-hat .* X-hat)) (:197-203), G2 = DX and sum |X|
+    // for the initial objective in the same pass
+    if (X0) CU_TRY(c, cudaMemcpyAsync(X, X0, LMN * 4, cudaMemcpyHostToDevice, s));
+    ST_TRY(init_x(c, X, !X0, seed, c->dred + kInitParts, &c->absx_init));
     // d = real(ifft(d-hat)) with d-hat = D-hat broadcast (CDL_setup.jl:207-210); the duals
     // g1, g3 start at zero (CDL_setup.jl:220-230).  In the spectral form nothing reads
     // these time-domain arrays before a D-step replaces them: written when first read.
@@ -973,20 +916,8 @@ int admm_init(cdlgb_ctx* c, const float* X0, const float* D0, uint64_t seed) {
         CU_TRY(c, cudaMemsetAsync(c->g1h, 0, nmf * 8, s));
         CU_TRY(c, cudaMemsetAsync(c->Dg, 0, (size_t)M * c->F * 8, s));
     }
-    // DX = real(ifft(sum_m D-hat .* X-hat)) (CDL_setup.jl:197-203); G2 = DX
-    for (int n0 = 0; n0 < N; n0 += c->chunk) {
-        const int cn = std::min(c->chunk, N - n0);
-        ST_TRY(r2c(c, (long long)M * cn, X + (size_t)n0 * M * Lg, c->sAh, M));
-        size_t FN = (size_t)c->F * cn;
-        k_spec_dot<<<(unsigned)((FN + 255) / 256), 256, 0, s>>>(c->sAh, c->G1h, c->sVh + (size_t)n0 * c->F,
-                                                              c->F, M, cn, 1.f / (float)Lg);
-        LAUNCH_CHECK(c, "k_spec_dot");
-    }
-    ST_TRY(c2r(c, N, c->sVh, c->DX, 1));
-    CU_TRY(c, cudaMemcpyAsync(c->G2, c->DX, LN * 4, cudaMemcpyDeviceToDevice, s));
     c->initialized = true;
     double obj = 0;
-    c->absx_init = 1;           // dred[0, 304) = k_init_x's sums of |X|, consumed here
     ST_TRY(admm_objective(c, &obj));
     c->obj_best = obj;
     return CDLGB_OK;
@@ -1189,7 +1120,9 @@ static int objective_async(cdlgb_ctx* c) {
     const double* fp = nullptr;
     int nf = 0;
     if (c->absx_init) {
-        // sum |X| came with the initial X (k_init_x)
+        // sum |X| came with the initial X (init_x)
+        pa = c->dred + kInitParts;
+        nb1 = c->absx_init;
         c->absx_init = 0;
     } else if (c->absx_fused && (c->xconv ? xconv_absx(c->xconv, &fp, &nf) : fused_absx(c, &fp, &nf))) {
         // sum |X| came with the last fused X-step

@@ -88,7 +88,7 @@ struct cdlgb_ctx {
     // with dspec: d, g1, g3 still to receive their initial values (d = G1 broadcast,
     // g1 = g3 = 0), written when first read, unless a D-step comes first
     int time_init = 0;
-    int absx_init = 0;              // dred[0, 304) holds sum |X| of the initial X
+    int absx_init = 0;              // partial sums of the initial |X| kept in dred (init.cu), else 0
     // LN state
     float *Y1 = nullptr, *y1 = nullptr, *DX = nullptr, *Td = nullptr, *G2 = nullptr, *g2 = nullptr;
     // LM state
@@ -197,6 +197,8 @@ void host_scalars_put(double* p);
 int admm_alloc(cdlgb_ctx* c);
 void admm_free(cdlgb_ctx* c);
 int admm_init(cdlgb_ctx* c, const float* X0, const float* D0, uint64_t seed);
+int init_d(cdlgb_ctx* c, uint64_t seed);                                    // init.cu
+int init_x(cdlgb_ctx* c, float* X, bool draw, uint64_t seed, double* out, int* np);
 int admm_code_update(cdlgb_ctx* c, int iters);
 int admm_dict_update(cdlgb_ctx* c, int iters);
 int admm_objective(cdlgb_ctx* c, double* obj);      // synchronous: result on host
