@@ -849,6 +849,15 @@ static int write_time_init(cdlgb_ctx* c) {
     return CDLGB_OK;
 }
 
+// the initial y2 = y3 = 0, for readers other than the X-steps that take them as zero
+int admm_write_duals(cdlgb_ctx* c) {
+    if (!c->zero_duals) return CDLGB_OK;
+    CU_TRY(c, cudaMemsetAsync(c->y2, 0, c->LMN * 4, c->stream));
+    CU_TRY(c, cudaMemsetAsync(c->y3, 0, c->LMN * 4, c->stream));
+    c->zero_duals = 0;
+    return CDLGB_OK;
+}
+
 int admm_init(cdlgb_ctx* c, const float* X0, const float* D0, uint64_t seed) {
     cudaStream_t s = c->stream;
     const int Lg = c->Lg, M = c->M, N = c->N, flen = 4 * c->p.filter_size;
@@ -891,10 +900,13 @@ int admm_init(cdlgb_ctx* c, const float* X0, const float* D0, uint64_t seed) {
         CU_TRY(c, cudaMemcpyAsync(c->dsum, c->G1, LM * 4, cudaMemcpyDeviceToDevice, s));
     }
     // X0 (CDL_setup.jl:191-192): given, or standard normal; masked to the 4-stride; with
-    // y2 = y3 = 0, DX = real(ifft(sum_m D-hat .* X-hat)) (:197-203), G2 = DX and sum |X|
+    // DX = real(ifft(sum_m D-hat .* X-hat)) (:197-203), G2 = DX and sum |X|
     // for the initial objective in the same pass
     if (X0) CU_TRY(c, cudaMemcpyAsync(X, X0, LMN * 4, cudaMemcpyHostToDevice, s));
     ST_TRY(init_x(c, X, !X0, seed, c->dred + kInitParts, &c->absx_init));
+    // y2 = y3 = 0 (CDL_setup.jl:220-230): the first X-step takes them as zero instead of
+    // reading them, where its kernel can; written when anything else reads them first
+    c->zero_duals = 1;
     // d = real(ifft(d-hat)) with d-hat = D-hat broadcast (CDL_setup.jl:207-210); the duals
     // g1, g3 start at zero (CDL_setup.jl:220-230).  In the spectral form nothing reads
     // these time-domain arrays before a D-step replaces them: written when first read.
@@ -909,13 +921,10 @@ int admm_init(cdlgb_ctx* c, const float* X0, const float* D0, uint64_t seed) {
     CU_TRY(c, cudaMemsetAsync(c->g2, 0, LN * 4, s));
     CU_TRY(c, cudaMemsetAsync(c->Td, 0, LN * 4, s));
     ST_TRY(refresh_G1h(c));
-    // spectral D-step: d-hat = D-hat broadcast, g1-hat = g3-hat = 0
-    if (c->dspec) {
-        const size_t nmf = (size_t)N * M * c->F;
-        ST_TRY(dspec_bcast(c, c->Dhs, c->G1h));
-        CU_TRY(c, cudaMemsetAsync(c->g1h, 0, nmf * 8, s));
-        CU_TRY(c, cudaMemsetAsync(c->Dg, 0, (size_t)M * c->F * 8, s));
-    }
+    // spectral D-step: d-hat = D-hat for every sequence and g1-hat = g3-hat = 0; the first
+    // D-step takes them from G1-hat (nothing else reads them), and writes both
+    c->spec_init = c->dspec;
+    if (c->dspec) CU_TRY(c, cudaMemsetAsync(c->Dg, 0, (size_t)M * c->F * 8, s));
     c->initialized = true;
     double obj = 0;
     ST_TRY(admm_objective(c, &obj));
@@ -934,6 +943,7 @@ int admm_code_update(cdlgb_ctx* c, int iters) {
         float* Xout = c->best_is_cur ? c->Xb[1 - c->xcur] : Xin;
         if (c->xconv) ST_TRY(xconv_xsteps(c, c->xconv, Xin, Xout, iters, c->N));
         else ST_TRY(fused_xsteps(c, Xin, Xout, iters));
+        c->zero_duals = 0;
         c->absx_fused = 1;
         if (Xout != Xin) {
             c->xcur = 1 - c->xcur;
@@ -949,6 +959,7 @@ int admm_code_update(cdlgb_ctx* c, int iters) {
         cdlgb_phase_end_n(c, PH_XSTEP, iters);
         return CDLGB_OK;
     }
+    if (iters > 0) ST_TRY(admm_write_duals(c));
     for (int it = 0; it < iters; ++it) {
         cdlgb_phase_begin(c, PH_XSTEP);
         // X_best aliases the current buffer: write the new X into the other one
@@ -997,6 +1008,7 @@ int admm_dict_update(cdlgb_ctx* c, int iters) {
     cudaStream_t s = c->stream;
     const size_t LN = c->LN, LM = c->LM;
     const int F = c->F, M = c->M, N = c->N, Lg = c->Lg;
+    if (!c->dspec && iters > 0) ST_TRY(admm_write_duals(c));
     for (int it = 0; it < iters; ++it) {
         cdlgb_phase_begin(c, PH_DSTEP);
         if (c->dspec) {
@@ -1026,6 +1038,7 @@ int admm_dict_update(cdlgb_ctx* c, int iters) {
                 ST_TRY(dspec_launch(c, c->sAh, c->G3h, n0, n0 + cn, slot0));
                 slot0 += dspec_nsub(cn, F, c->nsm);
             }
+            c->spec_init = 0;
             if (c->res_on) ST_TRY(resid_d_from_spec_parts(c, slot0 * ((F + 31) / 32)));
             ST_TRY(c2r(c, N, c->sVh, c->Td, 1));
             k_dg2<<<grid_for(LN, kBlock), kBlock, 0, s>>>(c->Td, c->g2, c->G2, c->S, Lg, c->L4,

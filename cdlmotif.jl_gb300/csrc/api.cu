@@ -539,6 +539,7 @@ int cdlgb_get(cdlgb_ctx* c, int32_t field, void* dst, size_t bytes) {
     if (!dst) return cdlgb_seterr(c, CDLGB_EINVAL, "dst is NULL");
     if (field == CDLGB_FIELD_D || field == CDLGB_FIELD_G1_DUAL || field == CDLGB_FIELD_G3_DUAL)
         ST_TRY(admm_sync_time_state(c));
+    if (field == CDLGB_FIELD_Y2_DUAL || field == CDLGB_FIELD_Y3_DUAL) ST_TRY(admm_write_duals(c));
     const void* src = nullptr;
     size_t want = 0;
     const size_t LMN = c->LMN * 4, LN = c->LN * 4, LM = c->LM * 4;
@@ -590,6 +591,7 @@ int cdlgb_autotune(cdlgb_ctx* c, int32_t max_candidates, double* ms_per_xstep, i
     if (!ms_per_xstep || !kind || !cluster || !filters || !n_candidates || !chosen || max_candidates <= 0)
         return cdlgb_seterr(c, CDLGB_EINVAL, "autotune: bad arguments");
     if (!c->fused) return cdlgb_seterr(c, CDLGB_ENOTSUP, "autotune: the cuFFT path has no variants");
+    ST_TRY(admm_write_duals(c));
     return fused_autotune(c, max_candidates, ms_per_xstep, kind, cluster, filters, n_candidates, chosen);
 }
 

@@ -85,9 +85,11 @@ struct cdlgb_ctx {
     // sums and their total are scratch
     float2 *g1h = nullptr, *Dg = nullptr, *G3h = nullptr, *spart = nullptr, *sumspec = nullptr;
     int dspec = 0, time_stale = 0;
+    int spec_init = 0;              // d-hat is still G1-hat for every sequence and g1-hat zero: not written
     // with dspec: d, g1, g3 still to receive their initial values (d = G1 broadcast,
     // g1 = g3 = 0), written when first read, unless a D-step comes first
     int time_init = 0;
+    int zero_duals = 0;             // y2 = y3 = 0 still, not written (admm_write_duals)
     int absx_init = 0;              // partial sums of the initial |X| kept in dred (init.cu), else 0
     // LN state
     float *Y1 = nullptr, *y1 = nullptr, *DX = nullptr, *Td = nullptr, *G2 = nullptr, *g2 = nullptr;
@@ -197,6 +199,7 @@ void host_scalars_put(double* p);
 int admm_alloc(cdlgb_ctx* c);
 void admm_free(cdlgb_ctx* c);
 int admm_init(cdlgb_ctx* c, const float* X0, const float* D0, uint64_t seed);
+int admm_write_duals(cdlgb_ctx* c);
 int init_d(cdlgb_ctx* c, uint64_t seed);                                    // init.cu
 int init_x(cdlgb_ctx* c, float* X, bool draw, uint64_t seed, double* out, int* np);
 int admm_code_update(cdlgb_ctx* c, int iters);
@@ -332,7 +335,6 @@ int dspec_slots(int N, int chunk, int F, int nsm);
 int dspec_launch(cdlgb_ctx* c, const float2* Yh, const float2* G3h, int c0, int c1, int slot0);
 int dspec_sums(cdlgb_ctx* c, const float2* G3h, float2* out);
 int dspec_g3(cdlgb_ctx* c, float2* dst, const float2* g1h, size_t rows);
-int dspec_bcast(cdlgb_ctx* c, float2* dst, const float2* plane);
 int dspec_scale(cdlgb_ctx* c, float* x, size_t n, float s);
 int admm_sync_time_state(cdlgb_ctx* c);
 // ---- background.cu ----

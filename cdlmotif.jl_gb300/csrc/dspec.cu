@@ -55,8 +55,10 @@ constexpr int kArr = 3;      // staged spectra: Y3-hat, g1-hat, d-hat
 // [c0, c1), in order, and writes that sub-range's sums to slot slot0 + s; warp w owns
 // filters w, w + 16, ...  With PIPE, each thread's spectra of sequence n + 1 are copied
 // to shared memory (asynchronous copies, two buffers) while sequence n is computed.
-// RES: also the residual partials (compiled out when false)
-template <int MW, bool PIPE, bool RES>
+// RES: also the residual partials (compiled out when false).  INIT: the first D-step of a
+// training, whose d-hat is G1-hat for every sequence and whose g1-hat is zero: neither is
+// read (two thirds of the loads), nor was it written
+template <int MW, bool PIPE, bool RES, bool INIT>
 __global__ void __launch_bounds__(kBins * kWarps, 1) k_dspec(SArgs A) {
     extern __shared__ float4 sm4[];
     const int M = A.M, F = A.F;
@@ -106,6 +108,7 @@ __global__ void __launch_bounds__(kBins * kWarps, 1) k_dspec(SArgs A) {
             const int m = min(w + kWarps * k, M - 1);
             float2* d0 = stg + ((size_t)(buf * kArr + 0) * MW + k) * nt + tid;
             __pipeline_memcpy_async(d0, A.Yh + ybase + (size_t)m * F, sizeof(float2));
+            if (INIT) continue;
             __pipeline_memcpy_async(d0 + (size_t)MW * nt, A.g1h + base + (size_t)m * F, sizeof(float2));
             __pipeline_memcpy_async(d0 + (size_t)2 * MW * nt, A.Dh + base + (size_t)m * F, sizeof(float2));
         }
@@ -132,6 +135,7 @@ __global__ void __launch_bounds__(kBins * kWarps, 1) k_dspec(SArgs A) {
             for (int k = 0; k < MW; ++k) {
                 const float2* s0 = stg + ((size_t)(buf * kArr + 0) * MW + k) * nt + tid;
                 yv[k] = s0[0];
+                if (INIT) continue;
                 g1v[k] = s0[(size_t)MW * nt];
                 dv[k] = s0[(size_t)2 * MW * nt];
             }
@@ -142,8 +146,16 @@ __global__ void __launch_bounds__(kBins * kWarps, 1) k_dspec(SArgs A) {
             for (int k = 0; k < MW; ++k) {
                 const int m = min(w + kWarps * k, M - 1);  // in bounds; unused when m >= M
                 yv[k] = A.Yh[ybase + (size_t)m * F];
+                if (INIT) continue;
                 g1v[k] = A.g1h[base + (size_t)m * F];
                 dv[k] = A.Dh[base + (size_t)m * F];
+            }
+        }
+        if (INIT) {
+#pragma unroll
+            for (int k = 0; k < MW; ++k) {
+                g1v[k] = make_float2(0.f, 0.f);
+                dv[k] = G1s[min(w + kWarps * k, M - 1) * kBins + lane];
             }
         }
         float2 hv[MW];
@@ -289,14 +301,6 @@ __global__ void k_dg_update(float2* __restrict__ Dg, const float2* __restrict__ 
     Dg[i] = cadd2(Dg[i], csub2(G3h[i], G1h[i]));
 }
 
-// broadcast of an (M, F) spectrum over n
-__global__ void k_bcast_spec(float2* __restrict__ dst, const float2* __restrict__ plane, size_t mf,
-                             size_t n) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-         i += (size_t)gridDim.x * blockDim.x)
-        dst[i] = plane[i % mf];
-}
-
 // dst = a - plane, the plane broadcast over n (g3-hat = g1-hat - Dg)
 __global__ void k_sub_bcast(float2* __restrict__ dst, const float2* __restrict__ a,
                             const float2* __restrict__ plane, size_t mf, size_t n) {
@@ -354,11 +358,13 @@ int dspec_launch(cdlgb_ctx* c, const float2* Yh, const float2* G3h, int c0, int 
     if (c->M <= 4 * kWarps) {
         // + the two staging buffers: 2 x 3 spectra x 4 filters x 512 threads
         const size_t smp = sm + (size_t)2 * kArr * 4 * kBins * kWarps * sizeof(float2);
-        auto k = c->res_on ? k_dspec<4, true, true> : k_dspec<4, true, false>;
+        auto k = c->res_on ? (c->spec_init ? k_dspec<4, true, true, true> : k_dspec<4, true, true, false>)
+                           : (c->spec_init ? k_dspec<4, true, false, true> : k_dspec<4, true, false, false>);
         CU_TRY(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smp));
         k<<<g, kBins * kWarps, smp, c->stream>>>(a);
     } else {
-        auto k = c->res_on ? k_dspec<8, false, true> : k_dspec<8, false, false>;
+        auto k = c->res_on ? (c->spec_init ? k_dspec<8, false, true, true> : k_dspec<8, false, true, false>)
+                           : (c->spec_init ? k_dspec<8, false, false, true> : k_dspec<8, false, false, false>);
         if (sm > 48 * 1024) CU_TRY(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
         k<<<g, kBins * kWarps, sm, c->stream>>>(a);
     }
@@ -374,13 +380,6 @@ int dspec_sums(cdlgb_ctx* c, const float2* G3h, float2* out) {
     k_dspec_sum<<<(unsigned)((4 * 2 * mf + 255) / 256), 256, 0, c->stream>>>(
         c->spart, c->Dg, out, mf, c->dslots, c->N, 1.0 / (double)c->Lg);
     LAUNCH_CHECK(c, "k_dspec_sum");
-    return CDLGB_OK;
-}
-
-int dspec_bcast(cdlgb_ctx* c, float2* dst, const float2* plane) {
-    const size_t mf = (size_t)c->M * c->F;
-    k_bcast_spec<<<grid_for(mf * c->N, 256), 256, 0, c->stream>>>(dst, plane, mf, mf * c->N);
-    LAUNCH_CHECK(c, "k_bcast_spec");
     return CDLGB_OK;
 }
 

@@ -67,8 +67,6 @@ __global__ void k_init_d(uint64_t seed, int Lg, int T, float* __restrict__ a, fl
 
 struct XArgs {
     float4* X;              // (N, M, La)
-    float4* y2;
-    float4* y3;
     const float4* G1;       // (M, La): taps b < W, zero after them
     float4* DX;             // (N, La)
     float4* G2;
@@ -104,8 +102,7 @@ __device__ __forceinline__ float2 unpack(unsigned long long a) {
 
 // X (CDL_setup.jl:191-192): standard normal on the rows l % 4 == 0, float4 j of (N, M, La)
 // from counter 4 j of the seed's splitmix64 stream (Box-Muller on two 24-bit uniforms); a
-// given X is masked to those rows instead (!DRAW).  y2 = y3 = 0 (CDL_setup.jl:220-230),
-// DX and G2 = DX (:197-203).
+// given X is masked to those rows instead (!DRAW).  DX and G2 = DX (CDL_setup.jl:197-203).
 //
 // A CTA takes ranges of RA values of a of one sequence, MG filters at a time: each warp
 // fills whole rows (with the values before the range that the taps reach, drawn again),
@@ -153,8 +150,6 @@ __global__ void __launch_bounds__(kNT, 3) k_init_x(XArgs A) {
                             }
                             if (i >= Hp && t0 == 0) {      // the range's own
                                 A.X[j] = make_float4(v, 0.f, 0.f, 0.f);
-                                A.y2[j] = z;
-                                A.y3[j] = z;
                                 // sum |X| as a compensated pair (two-sum)
                                 const float x = fabsf(v), t = __fadd_rn(s, x), b = __fsub_rn(t, s);
                                 sc = __fadd_rn(sc, __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(x, b)));
@@ -251,10 +246,10 @@ int init_d(cdlgb_ctx* c, uint64_t seed) {
     return CDLGB_OK;
 }
 
-// X (drawn, or masked where it stands), y2, y3, DX, G2 from G1; *np partial sums of |X| in out
+// X (drawn, or masked where it stands), DX, G2 from G1; *np partial sums of |X| in out
 int init_x(cdlgb_ctx* c, float* X, bool draw, uint64_t seed, double* out, int* np) {
     XArgs a;
-    a.X = (float4*)X; a.y2 = (float4*)c->y2; a.y3 = (float4*)c->y3; a.G1 = (const float4*)c->G1;
+    a.X = (float4*)X; a.G1 = (const float4*)c->G1;
     a.DX = (float4*)c->DX; a.G2 = (float4*)c->G2; a.out = out; a.seed = seed;
     a.N = c->N; a.M = c->M; a.La = c->Lg / 4; a.W = c->p.filter_size;
     // A range per CTA: a thread per 8 values, times as many filters at a time as fill the

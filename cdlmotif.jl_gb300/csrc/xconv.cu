@@ -69,6 +69,7 @@ struct Args {
     const float2* Hsd;      // [n/2 + 1] (H[k] + H[n-k])/2n, (H[k] - H[n-k])/2n
     int n0, M, Lg, L4, gamma, iters, T, G;
     int first, last;        // k_xc_solve: the code update's first, last X-step
+    int zero;               // y2, y3 are zero and not written yet (the initial state)
     float lam, rho, kc;
     int NB;                 // blocks of 16 taps (the last one filled up with zeros)
     int B, CG, nchunk;      // pairs per CTA, row blocks per warp, row blocks
@@ -348,7 +349,9 @@ __device__ __forceinline__ float codes(const Args& A, const float4* gs, const fl
                 const float* src = (MODE == FIRST ? A.Xin : A.V) + ra[u];
                 xa[u] = on ? *reinterpret_cast<const float4*>(src) : z4;
                 xb[u] = two ? *reinterpret_cast<const float4*>(src + Lg) : z4;
-                if (MODE != LAST) {
+                if (MODE == FIRST && A.zero) {
+                    aa[u] = ab[u] = ba[u] = bb[u] = z4;
+                } else if (MODE != LAST) {
                     aa[u] = on ? *reinterpret_cast<const float4*>(A.y2 + ra[u]) : z4;
                     ba[u] = on ? *reinterpret_cast<const float4*>(A.y3 + ra[u]) : z4;
                     ab[u] = two ? *reinterpret_cast<const float4*>(A.y2 + ra[u] + Lg) : z4;
@@ -915,7 +918,7 @@ int xconv_xsteps(cdlgb_ctx* c, void* p, const float* Xin, float* Xout, int iters
     a.T = 4 * c->p.filter_size; a.G = s.G;
     a.lam = c->p.lambda; a.rho = c->p.rho; a.kc = c->p.sherman_const_csc;
     a.NB = s.NB; a.B = s.B; a.CG = s.CG; a.nchunk = s.nchunk; a.pitch = s.pitch;
-    a.n = P->n; a.nst = P->nst;
+    a.n = P->n; a.nst = P->nst; a.zero = c->zero_duals;
     for (int i = 0; i < P->nst; ++i) { a.radix[i] = P->radix[i]; a.twoff[i] = P->twoff[i]; }
     // the fused kernel's timer, in X-steps, where a fused form exists for the size
     if (c->fused) cdlgb_phase_begin(c, PH_XFUSED);

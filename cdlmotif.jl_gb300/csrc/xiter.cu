@@ -144,6 +144,7 @@ void* iter_plan_create_nth(cdlgb_ctx* c, int nth, int want_cs, int* status) {
     }
     if (!P) return nullptr;
     std::vector<float2> tw2 = regfft_twiddles(v->N1, v->P);
+    tw2.resize((size_t)2 * c->Lg, make_float2(0.f, 0.f));          // and 2 Lg zeros after them
     cudaError_t e = v->tables();
     if (e == cudaSuccess) e = dev_copy_in(c, (void**)&P->tw2, tw2.data(), tw2.size() * sizeof(float2));
     // process-wide per kernel: the same cap for every context
@@ -213,6 +214,7 @@ int iter_xsteps_n(cdlgb_ctx* c, void* p, const float* Xin, float* Xout, int iter
     a.res_part = P->res_part;
     a.N = Nlim; a.M = c->M; a.L4 = c->L4; a.gamma = c->gamma; a.iters = iters;
     a.lam = c->p.lambda; a.rho = c->p.rho; a.kc = c->p.sherman_const_csc;
+    a.zeros = c->zero_duals ? reinterpret_cast<const float*>(P->tw2 + c->Lg) : nullptr;
     a.ld = P->ld; a.ld3 = P->ld3;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];

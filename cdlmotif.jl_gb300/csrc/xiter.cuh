@@ -50,6 +50,7 @@ struct IArgs {
     double* res_part;       // per CTA: the five X-step residual sums of the final iterate
     int N, M, L4, gamma, iters;
     float lam, rho, kc;
+    const float* zeros;     // [2 Lg], read in place of y2, y3 while these are zero and not written; else null
     int ld, ld3;            // row strides (pairs) of the y2 and compacted y3 rows in shared memory
 };
 
@@ -140,6 +141,7 @@ __device__ __forceinline__ void prefetch_next(const IArgs& A, int n, int m0, int
     const size_t r0 = ((size_t)n * A.M + m0) * Lg;
     for (int q = lane; q < 3 * MC + 4; q += 32) {
         if (q < 3 * MC) {
+            if (A.zeros && q >= MC) continue;
             const float* base = q < MC ? A.Xin : q < 2 * MC ? A.y2 : A.y3;
             l2_prefetch(base + r0 + (size_t)(q % MC) * Lg, rb);
         } else if (q < 3 * MC + 3) {
@@ -237,11 +239,13 @@ __global__ void __launch_bounds__(NT, MINB) k_xiter(IArgs A) {
         // the HBM loads need no register array)
         if (pair) {
             const size_t ra = ((size_t)n * M + m0 + 2 * grp) * Lg + gl;
+            const float* y2r = A.zeros ? A.zeros + gl : A.y2 + ra;
+            const float* y3r = A.zeros ? A.zeros + gl : A.y3 + ra;
 #pragma unroll 16
             for (int n2 = 0; n2 < P; ++n2) {
                 const int o = N1 * n2;
-                float2 a2 = f2(A.y2[ra + o], A.y2[ra + Lg + o]);
-                float2 a3 = f2(A.y3[ra + o], A.y3[ra + Lg + o]);
+                float2 a2 = f2(y2r[o], y2r[Lg + o]);
+                float2 a3 = f2(y3r[o], y3r[Lg + o]);
                 const float2 V = xprep2(f2(A.Xin[ra + o], A.Xin[ra + Lg + o]), a2, a3, lam, keep);
                 y2p[o] = a2;
                 if (!keep) y3p[W3 * n2] = a3;
