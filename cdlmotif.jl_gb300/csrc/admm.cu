@@ -159,15 +159,15 @@ __global__ void k_dprep(const float4* __restrict__ X, const float4* __restrict__
     }
 }
 
-// Y3 = projectionX!(X + y3) (csc_kernels.jl:68-82) of a chunk, for the spectral D-step on
-// lengths without the streaming transforms: X + 0 on the rows l % 4 == 0 (every row
-// starts at a multiple of 4 floats, so those are the .x lanes), where every X-step
-// leaves y3 = +0 exactly (projectionX! keeps X + y3 there, so y3' = (y3 + X) - Y3 = +0,
-// as initialisation sets it), and 0 on the others -- the values k_dfwd transforms.
-__global__ void k_y3(const float4* __restrict__ X, float4* __restrict__ Y3, size_t n4) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n4;
+// The kept rows of Y3 = projectionX!(X + y3) (csc_kernels.jl:68-82) of a chunk, for the
+// spectral D-step on lengths without the streaming transforms: X + 0 on the rows
+// l % 4 == 0 (every row starts at a multiple of 4 floats, so those are the .x lanes),
+// where every X-step leaves y3 = +0 exactly (projectionX! keeps X + y3 there, so
+// y3' = (y3 + X) - Y3 = +0, as initialisation sets it) -- the values k_y3fwd transforms.
+__global__ void k_y3(const float4* __restrict__ X, float* __restrict__ Y3, size_t n) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
          i += (size_t)gridDim.x * blockDim.x)
-        Y3[i] = make_float4(X[i].x + 0.f, 0.f, 0.f, 0.f);
+        Y3[i] = X[i].x + 0.f;
 }
 
 __global__ void k_sub(const float* __restrict__ a, const float* __restrict__ b,
@@ -561,22 +561,23 @@ double host_uniform(uint64_t seed, uint64_t i) {
 struct PlanEntry { int dir; long long batch; cufftHandle h; void* work; };
 typedef std::vector<PlanEntry> PlanCache;
 
-// R2C (dir 0) or C2R (dir 1) plan of length Lg over `batch` contiguous columns
+// R2C (dir 0) or C2R (dir 1) plan of length Lg, or R2C of length Lg / 4 (dir 2), over `batch` contiguous columns
 int get_plan(cdlgb_ctx* c, int dir, long long batch, cufftHandle* out) {
     if (!c->plans) c->plans = new PlanCache();
     PlanCache& pc = *(PlanCache*)c->plans;
     for (auto& e : pc)
         if (e.dir == dir && e.batch == batch) { *out = e.h; return CDLGB_OK; }
-    long long n[1] = {c->Lg}, in_r[1] = {c->Lg}, in_c[1] = {c->F};
+    const long long len = dir == 2 ? c->Lg / 4 : c->Lg, bins = len / 2 + 1;
+    long long n[1] = {len}, in_r[1] = {len}, in_c[1] = {bins};
     size_t ws = 0;
     cufftHandle h;
     FFT_TRY(c, cufftCreate(&h));
     // the work area comes from the context's stream-ordered allocations, not from cuFFT
     FFT_TRY(c, cufftSetAutoAllocation(h, 0));
-    if (dir == 0)
-        FFT_TRY(c, cufftMakePlanMany64(h, 1, n, in_r, 1, c->Lg, in_c, 1, c->F, CUFFT_R2C, batch, &ws));
+    if (dir != 1)
+        FFT_TRY(c, cufftMakePlanMany64(h, 1, n, in_r, 1, len, in_c, 1, bins, CUFFT_R2C, batch, &ws));
     else
-        FFT_TRY(c, cufftMakePlanMany64(h, 1, n, in_c, 1, c->F, in_r, 1, c->Lg, CUFFT_C2R, batch, &ws));
+        FFT_TRY(c, cufftMakePlanMany64(h, 1, n, in_c, 1, bins, in_r, 1, len, CUFFT_C2R, batch, &ws));
     void* work = nullptr;
     int st = dev_alloc(c, &work, ws);
     if (st != CDLGB_OK) { cufftDestroy(h); return st; }
@@ -706,7 +707,7 @@ size_t admm_footprint(const cdlgb_params* p, int L4, int N, int fused) {
     if (spec) {
         // spectral D-step: the sums' slots and the Y3 half-spectra beyond the cuFFT chunk
         const size_t sch = spec_chunk_for(N, (int)M, (int)Lg), ch = chunk_for(N, (int)M, (int)Lg);
-        b += (size_t)dspec_slots(N, (int)sch, (int)F, device_sms()) * 2 * M * F * 8;
+        b += (size_t)dspec_slots(N, (int)sch, (int)M, (int)F, device_sms()) * 2 * M * F * 8;
         b += (sch - ch) * M * F * 8;
     }
     b += 8 * LN * 4;                            // Y1 y1 DX Td G2 g2 + 2 scratch
@@ -774,7 +775,7 @@ int admm_alloc(cdlgb_ctx* c) {
     c->nsm = device_sms();
     if (c->g1h) {
         c->schunk = spec_chunk_for(c->N, c->M, c->Lg);
-        c->dslots = dspec_slots(c->N, c->schunk, c->F, c->nsm);
+        c->dslots = dspec_slots(c->N, c->schunk, c->M, c->F, c->nsm);
         ST_TRY(A((void**)&c->spart, dspec_part_bytes(c->M, c->F, c->dslots)));
     }
     const size_t cLMN = (size_t)c->chunk * c->M * c->Lg, cSp = (size_t)c->chunk * c->M * c->F;
@@ -1022,21 +1023,24 @@ int admm_dict_update(cdlgb_ctx* c, int iters) {
             for (int n0 = 0; n0 < N; n0 += c->schunk) {
                 const int cn = std::min(c->schunk, N - n0);
                 if (fw) {
-                    ST_TRY(dfwd_run(c, fw, cur_X(c), n0, cn, c->sAh, nullptr, nullptr));
+                    ST_TRY(y3fwd_run(c, fw, cur_X(c), n0, cn, c->sAh));
                 } else {
-                    // lengths without the streaming transforms: Y3 formed in the time
-                    // domain and transformed, a cuFFT chunk at a time
+                    // lengths without the streaming transforms: Y3's kept rows gathered
+                    // and transformed, a cuFFT chunk at a time
                     for (int m0 = n0; m0 < n0 + cn; m0 += c->chunk) {
                         const int cm = std::min(c->chunk, n0 + cn - m0);
-                        const size_t cl = (size_t)cm * M * Lg;
-                        k_y3<<<grid_for(cl / 4, kBlock), kBlock, 0, s>>>(
-                            (const float4*)(cur_X(c) + (size_t)m0 * M * Lg), (float4*)c->sA, cl / 4);
+                        const size_t cl = (size_t)cm * M * (Lg / 4);
+                        k_y3<<<grid_for(cl, kBlock), kBlock, 0, s>>>(
+                            (const float4*)(cur_X(c) + (size_t)m0 * M * Lg), c->sA, cl);
                         LAUNCH_CHECK(c, "k_y3");
-                        ST_TRY(r2c(c, (long long)M * cm, c->sA, c->sAh + (size_t)(m0 - n0) * M * F, M));
+                        cufftHandle h;
+                        ST_TRY(get_plan(c, 2, (long long)M * cm, &h));
+                        FFT_TRY(c, cufftExecR2C(h, c->sA, c->sAh + (size_t)(m0 - n0) * M * (Lg / 8 + 1)));
+                        c->fft_calls++;
                     }
                 }
                 ST_TRY(dspec_launch(c, c->sAh, c->G3h, n0, n0 + cn, slot0));
-                slot0 += dspec_nsub(cn, F, c->nsm);
+                slot0 += dspec_nsub(cn, M, F, c->nsm);
             }
             c->spec_init = 0;
             if (c->res_on) ST_TRY(resid_d_from_spec_parts(c, slot0 * ((F + 31) / 32)));

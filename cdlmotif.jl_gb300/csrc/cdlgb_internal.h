@@ -273,6 +273,7 @@ int noalloc_warm_current_device();
 void* dfwd_plan_create(cdlgb_ctx* c, int* status);
 void dfwd_plan_free(cdlgb_ctx* c, void* p);
 int dfwd_run(cdlgb_ctx* c, void* p, const float* X, int n0, int cn, float2* Yh, float2* Hh, float2* Dh);
+int y3fwd_run(cdlgb_ctx* c, void* p, const float* X, int n0, int cn, float2* Yh);
 int dinv_run(cdlgb_ctx* c, void* p, const float2* Dh, int n0, int cn, float scale);
 // batched R2C / C2R of R contiguous rows on the register FFT (cuFFT's layouts and
 // scaling); two rows share a transform only inside a group of grp consecutive rows
@@ -330,8 +331,8 @@ void scan_free(cdlgb_ctx* c);
 // ---- dspec.cu ----
 int dspec_max_m();
 size_t dspec_part_bytes(int M, int F, int slots);
-int dspec_nsub(int cn, int F, int nsm);
-int dspec_slots(int N, int chunk, int F, int nsm);
+int dspec_nsub(int cn, int M, int F, int nsm);
+int dspec_slots(int N, int chunk, int M, int F, int nsm);
 int dspec_launch(cdlgb_ctx* c, const float2* Yh, const float2* G3h, int c0, int c1, int slot0);
 int dspec_sums(cdlgb_ctx* c, const float2* G3h, float2* out);
 int dspec_g3(cdlgb_ctx* c, float2* dst, const float2* g1h, size_t rows);

@@ -49,13 +49,13 @@ const std::vector<Variant>& all_variants() {
 }
 
 struct FwdPlan {
-    kern_t k;
+    kern_t k, ky;
     kinv_t ki;
     kr2c_t kf;
     kc2r_t kb;
     int N1, P;
-    size_t smem;
-    int grid, grid_inv, grid_rows_f, grid_rows_b;
+    size_t smem, smem_y;
+    int grid, grid_y, grid_inv, grid_rows_f, grid_rows_b;
     float2* tw2;
 };
 
@@ -71,10 +71,13 @@ void* dfwd_plan_create(cdlgb_ctx* c, int* status) {
         if (cand.N1 * cand.P == c->Lg) v = &cand;
     if (!v) return nullptr;
     FwdPlan* P = new FwdPlan();
-    P->k = v->k; P->ki = v->ki; P->kf = v->kf; P->kb = v->kb; P->N1 = v->N1; P->P = v->P;
+    P->k = v->k; P->ky = v->ky; P->ki = v->ki; P->kf = v->kf; P->kb = v->kb; P->N1 = v->N1; P->P = v->P;
     const int threads = 256, groups = (threads / 32) * (32 / v->N1);
     const size_t buf = ((size_t)v->P * (v->N1 + 1) + 1) & ~(size_t)1;
     P->smem = ((size_t)v->P * v->N1 + (size_t)groups * buf) * sizeof(float2);
+    // k_y3fwd: lane groups of N1 / 4, their buffers a multiple of 16 and N1 / 4 places apart
+    const int n1y = v->N1 / 4, rows = v->P * (n1y + 1);
+    P->smem_y = ((size_t)v->P * n1y + (size_t)4 * groups * (rows + (16 + n1y - rows % 16) % 16)) * sizeof(float2);
     std::vector<float2> tw2 = regfft_twiddles(v->N1, v->P);
     cudaError_t e = v->tables();
     if (e == cudaSuccess) e = dev_copy_in(c, (void**)&P->tw2, tw2.data(), tw2.size() * sizeof(float2));
@@ -82,12 +85,15 @@ void* dfwd_plan_create(cdlgb_ctx* c, int* status) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(P->ki, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(P->kf, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(P->kb, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(P->ky, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+    int per_sm_y = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_y, P->ky, threads, P->smem_y);
     int per_sm = 0, per_sm_inv = 0, per_sm_f = 0, per_sm_b = 0;
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, P->k, threads, P->smem);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_inv, P->ki, threads, P->smem);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_f, P->kf, threads, P->smem);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_b, P->kb, threads, P->smem);
-    if (e != cudaSuccess || per_sm < 1 || per_sm_inv < 1 || per_sm_f < 1 || per_sm_b < 1) {
+    if (e != cudaSuccess || per_sm < 1 || per_sm_y < 1 || per_sm_inv < 1 || per_sm_f < 1 || per_sm_b < 1) {
         *status = cdlgb_seterr(c, CDLGB_ECUDA, "D-step transform setup failed: %s",
                                e != cudaSuccess ? cudaGetErrorString(e) : "no CTA fits");
         dev_free(c, P->tw2);
@@ -98,6 +104,7 @@ void* dfwd_plan_create(cdlgb_ctx* c, int* status) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     P->grid = per_sm * sms;
+    P->grid_y = per_sm_y * sms;
     P->grid_inv = per_sm_inv * sms;
     P->grid_rows_f = per_sm_f * sms;
     P->grid_rows_b = per_sm_b * sms;
@@ -111,8 +118,18 @@ void dfwd_plan_free(cdlgb_ctx* c, void* p) {
     delete P;
 }
 
+// Y3-hat's bins 0 .. Lg/8 of sequences [n0, n0 + cn) into Yh, (cn, M, Lg/8 + 1)
+int y3fwd_run(cdlgb_ctx* c, void* p, const float* X, int n0, int cn, float2* Yh) {
+    FwdPlan* P = (FwdPlan*)p;
+    FArgs a = {};
+    a.X = X + (size_t)n0 * c->M * c->Lg; a.Yh = Yh; a.tw2 = P->tw2; a.cn = cn; a.M = c->M;
+    P->ky<<<P->grid_y, 256, P->smem_y, c->stream>>>(a);
+    LAUNCH_CHECK(c, "k_y3fwd");
+    return CDLGB_OK;
+}
+
 // Y3-hat, H-hat and d-hat of sequences [n0, n0 + cn) into Yh, Hh, Dh (chunk layout); a
-// null Hh or Dh skips that transform.
+// null Dh skips that transform.
 int dfwd_run(cdlgb_ctx* c, void* p, const float* X, int n0, int cn, float2* Yh, float2* Hh, float2* Dh) {
     FwdPlan* P = (FwdPlan*)p;
     const size_t off = (size_t)n0 * c->M * c->Lg;

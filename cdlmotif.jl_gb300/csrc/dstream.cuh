@@ -55,9 +55,9 @@ typedef void (*kern_t)(FArgs);
 typedef void (*kinv_t)(IArgsD);
 typedef void (*kr2c_t)(const float*, float2*, const float2*, long, int);
 typedef void (*kc2r_t)(const float2*, float*, const float2*, long, int);
-// one transform length: the forward D-step transforms, their inverse, the row R2C and
-// C2R; tables uploads the constant tables of the unit that instantiated them
-struct Variant { int N1, P; kern_t k; kinv_t ki; kr2c_t kf; kc2r_t kb; cudaError_t (*tables)(); };
+// one transform length: the forward D-step transforms, Y3's alone, their inverse, the row
+// R2C and C2R; tables uploads the constant tables of the unit that instantiated them
+struct Variant { int N1, P; kern_t k, ky; kinv_t ki; kr2c_t kf; kc2r_t kb; cudaError_t (*tables)(); };
 
 }  // namespace dstream
 
@@ -159,8 +159,63 @@ __global__ void __launch_bounds__(256, 2) k_dfwd(FArgs A) {
         const bool hb = ma + 1 < A.M;
         const int bo = hb ? Lg : 0, fo = hb ? F : 0;
         dfwd_one<N1, P, 0>(A, sb, gl, tw2, act, keep, bo, fo, ra, pa, oa);
-        if (A.Hh) dfwd_one<N1, P, 1>(A, sb, gl, tw2, act, keep, bo, fo, ra, pa, oa);   // uniform
-        if (A.Dh) dfwd_one<N1, P, 2>(A, sb, gl, tw2, act, keep, bo, fo, ra, pa, oa);
+        dfwd_one<N1, P, 1>(A, sb, gl, tw2, act, keep, bo, fo, ra, pa, oa);
+        if (A.Dh) dfwd_one<N1, P, 2>(A, sb, gl, tw2, act, keep, bo, fo, ra, pa, oa);   // uniform
+    }
+}
+
+// Y3 alone, for the spectral D-step.  Y3 is zero off the rows l % 4 == 0, so its transform is
+// that of the La = Lg / 4 kept rows, which repeats with period La: Y3-hat[f] = Z[f mod La],
+// and Z, of real rows, is given by its bins 0 .. La/2.  A lane group of N1 = 4 or 8 lanes
+// transforms the kept rows of a filter pair, lane n1 the rows n1 + N1 n2, and stores
+// those bins: a quarter of the arithmetic, of the shared memory and of the bytes written
+// (and read by the solve) that k_dfwd takes for it.  Bound by HBM, the lines of X being read
+// whole: 1.75 -> 0.85 ms (6.5 TB/s) for 20000 x 64 filters of 928 rows.  The groups' buffers start N1
+// places apart modulo 16: a half-warp's 8-byte accesses fall on distinct banks.
+template <int N1, int P>
+__global__ void __launch_bounds__(256, 2) k_y3fwd(FArgs A) {
+    constexpr int La = N1 * P, Lg = 4 * La;
+    constexpr int G = 32 / N1;
+    constexpr int RS = N1 + 1;
+    constexpr int BUF = P * RS + (16 + N1 - P * RS % 16) % 16;
+    constexpr int F = La / 2 + 1;
+    extern __shared__ float4 smem4[];
+    float2* tw2 = reinterpret_cast<float2*>(smem4);        // [P][N1]
+    float2* bufs = tw2 + P * N1;                           // [groups][BUF]
+    // exp(-2 pi i n1 k2 / La), from the table of Lg
+    for (int t = threadIdx.x; t < P * N1; t += blockDim.x) tw2[t] = A.tw2[4 * t];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int gw = (threadIdx.x >> 5) * G + lane / N1;
+    const int gl = lane % N1;
+    const int groups = (blockDim.x >> 5) * G;
+    float2* sb = bufs + (size_t)gw * BUF;
+    const int pairs = (A.M + 1) / 2;
+    const long items = (long)A.cn * pairs;
+    const long stride = (long)gridDim.x * groups;
+    const long rounds = (items + stride - 1) / stride;
+    for (long r = 0; r < rounds; ++r) {
+        const long item = r * stride + (long)blockIdx.x * groups + gw;
+        const bool act = item < items;
+        const long n = act ? item / pairs : 0;
+        const int ma = act ? 2 * (int)(item - n * pairs) : 0;
+        const bool hb = ma + 1 < A.M;                      // false: the last pair of an odd M
+        if (act) {
+            const float* x = A.X + ((size_t)n * A.M + ma) * Lg + 4 * gl;
+            const int bo = hb ? Lg : 0;
+            // X + 0 on the kept rows, as in dfwd_one
+#pragma unroll 16
+            for (int n2 = 0; n2 < P; ++n2)
+                sb[n2 * RS + gl] = f2(__ldg(x + 4 * N1 * n2) + 0.f, __ldg(x + bo + 4 * N1 * n2) + 0.f);
+            fwd_step1<N1, P>(sb, gl, tw2);
+        }
+        __syncwarp();
+        fwd_step2<N1, P>(sb, gl, act);
+        if (act) {
+            float2* o = A.Yh + ((size_t)n * A.M + ma) * F;
+            split_store<La, N1>(sb, gl, o, o + (hb ? F : 0));
+        }
+        __syncwarp();
     }
 }
 
@@ -357,4 +412,4 @@ __global__ void __launch_bounds__(256, 2) k_rows_c2r(const float2* __restrict__ 
 }  // namespace
 
 #define DSTREAM_VARIANT(N1, P) \
-    {N1, P, k_dfwd<N1, P>, k_dinv<N1, P>, k_rows_r2c<N1, P>, k_rows_c2r<N1, P>, regfft_upload_tables}
+    {N1, P, k_dfwd<N1, P>, k_y3fwd<N1 / 4, P>, k_dinv<N1, P>, k_rows_r2c<N1, P>, k_rows_c2r<N1, P>, regfft_upload_tables}

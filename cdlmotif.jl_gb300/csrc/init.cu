@@ -142,8 +142,8 @@ __global__ void __launch_bounds__(kNT, 3) k_init_x(XArgs A) {
                             const size_t j = row + a;
                             if (DRAW) {
                                 const uint64_t h = splitmix64(A.seed * 0x2545F4914F6CDD1Dull ^ (uint64_t)(4 * j));
-                                const float u1 = ((float)(h >> 40) + 0.5f) * (1.0f / 16777216.0f);
-                                const float u2 = ((float)(h & 0xFFFFFFull) + 0.5f) * (1.0f / 16777216.0f);
+                                const float u1 = ((float)(uint32_t)(h >> 40) + 0.5f) * (1.0f / 16777216.0f);
+                                const float u2 = ((float)((uint32_t)h & 0xFFFFFFu) + 0.5f) * (1.0f / 16777216.0f);
                                 v = sqrtf(-2.f * logf(u1)) * cospif(2.f * u2);
                             } else {
                                 v = A.X[j].x;
