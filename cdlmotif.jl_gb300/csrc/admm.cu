@@ -170,11 +170,12 @@ __global__ void k_y3(const float4* __restrict__ X, float* __restrict__ Y3, size_
         Y3[i] = X[i].x + 0.f;
 }
 
+// o = a - b, and m values of t behind the n
 __global__ void k_sub(const float* __restrict__ a, const float* __restrict__ b,
-                      float* __restrict__ o, size_t n) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+                      float* __restrict__ o, size_t n, const float* __restrict__ t, size_t m) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n + m;
          i += (size_t)gridDim.x * blockDim.x)
-        o[i] = a[i] - b[i];
+        o[i] = i < n ? a[i] - b[i] : t[i - n];
 }
 
 // Per (f, n): the Sherman-Morrison dictionary solve (cdl_kernels.jl:2-33, train.jl:52-61),
@@ -390,6 +391,18 @@ __global__ void k_abssum(const float4* __restrict__ X, size_t n4, double* __rest
     if (threadIdx.x == 0) out[blockIdx.x] = acc;
 }
 
+// Whether this block is the last of its grid to get here: its partial results and every
+// other block's are then visible to it.  counter returns to zero.
+__device__ __forceinline__ bool last_block(unsigned* counter) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(counter, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
 // Sums of many float32 terms.  A float64 sum per term is what bounds such a pass here (two
 // FP64 operations per SM and cycle: 13.2 ms for the threshold's two passes over 1.19e9
 // codes, 0.72 TB/s), so runs of 16 or 32 terms go into a compensated float32 pair first
@@ -416,11 +429,15 @@ __device__ __forceinline__ float add_dev2(float& s, float& c, float x, float mh,
 }
 constexpr float kDevMin = 1e-10f, kDevMax = 1e17f;     // deviations whose squares the pairs hold
 
-// sum over the data window of (DX - S)^2  (||W*DX - S||^2): rows of q4 float4s, window rows
-// at gamma / 4 of the row of Lg / 4
+// The objective: the sum over the data window of (DX - S)^2  (||W*DX - S||^2; rows of q4
+// float4s, window rows at gamma / 4 of the row of Lg / 4) into out by blocks; the last block
+// adds those and the nb1 partial sums of |X| at pa and writes 0.5 fit + lam |X| to obj, which
+// is pinned host memory: one launch where there were two and a copy (31 -> 22 us with the
+// wait at 200 sequences of 232 rows, of which the sums take 2).
 constexpr int kFitBlocks = 152 * 4;
 __global__ void k_fit(const float4* __restrict__ DX, const float4* __restrict__ S, unsigned Lg4, unsigned q4,
-                      unsigned g4, size_t n4, double* __restrict__ out) {
+                      unsigned g4, size_t n4, double* out, const double* __restrict__ pa, int nb1, double lam,
+                      unsigned* counter, double* obj) {
     __shared__ double sh[32];
     double acc = 0.0;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -459,32 +476,29 @@ __global__ void k_fit(const float4* __restrict__ DX, const float4* __restrict__ 
     }
     acc = block_sum_d(acc, sh);
     if (threadIdx.x == 0) out[blockIdx.x] = acc;
-}
-
-// out[0] = 0.5 * sum(pb[0..nb2)) + lam * sum(pa[0..nb1))
-__global__ void k_obj_final(const double* __restrict__ pa, int nb1, const double* __restrict__ pb,
-                            int nb2, double lam, double* __restrict__ out) {
-    __shared__ double sh[32];
+    if (!last_block(counter)) return;
     double a = 0.0, b = 0.0;
     for (int i = threadIdx.x; i < nb1; i += blockDim.x) a += pa[i];
-    for (int i = threadIdx.x; i < nb2; i += blockDim.x) b += pb[i];
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) b += __ldcg(out + i);
     a = block_sum_d(a, sh);
     b = block_sum_d(b, sh);
-    if (threadIdx.x == 0) out[0] = 0.5 * b + lam * a;
+    if (threadIdx.x == 0) *obj = 0.5 * b + lam * a;
 }
 
 // std of the positive entries: pass 1 (mu null) count + sum, pass 2 sum of squared
 // deviations from mu; 32 entries per run.  N = 20000, L = 200, K = 64 (4.75 GB a pass):
-// 13.2 ms for both passes with a float64 sum per entry, 2.2 ms with the runs.
+// 13.2 ms for both passes with a float64 sum per entry, 2.65 ms with the runs.  The last block
+// adds the partial sums: the count and mean to stat, or the deviation to the pinned host
+// scalar dev (two launches and a copy less: 48 -> 29 us with the wait at 200 x 10 x 232).
 constexpr int kPosBlocks = 152 * 4;
 template <bool SECOND>
 __global__ void __launch_bounds__(256) k_pos_stats(const float4* __restrict__ X, size_t n4,
-                                                   const double* __restrict__ mu, double* __restrict__ out) {
+                                                   double* out, double* stat, unsigned* counter, double* dev) {
     __shared__ double sh[32];
     constexpr int U = 8;
     double acc = 0.0;
     unsigned count = 0;
-    const double m = SECOND ? mu[0] : 0.0;
+    const double m = SECOND ? stat[1] : 0.0;
     const float mh = (float)m, ml = (float)(m - (double)mh);
     const bool mean_ok = fabsf(mh) <= kDevMax;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -534,21 +548,17 @@ __global__ void __launch_bounds__(256) k_pos_stats(const float4* __restrict__ X,
         out[2 * blockIdx.x] = n;
         out[2 * blockIdx.x + 1] = acc;
     }
-}
-
-__global__ void k_pos_final(const double* __restrict__ part, int nb, double* __restrict__ out,
-                            int second) {
-    __shared__ double sh[32];
+    if (!last_block(counter)) return;
     double c = 0.0, s = 0.0;
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-        c += part[2 * i];
-        s += part[2 * i + 1];
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
+        c += __ldcg(out + 2 * i);
+        s += __ldcg(out + 2 * i + 1);
     }
     c = block_sum_d(c, sh);
     s = block_sum_d(s, sh);
     if (threadIdx.x == 0) {
-        if (!second) { out[0] = c; out[1] = c > 0 ? s / c : 0.0; }
-        else out[2] = out[0] > 1 ? sqrt(s / (out[0] - 1.0)) : nan("");
+        if (!SECOND) { stat[0] = c; stat[1] = c > 0 ? s / c : 0.0; }
+        else *dev = stat[0] > 1 ? sqrt(s / (stat[0] - 1.0)) : nan("");
     }
 }
 
@@ -680,6 +690,14 @@ int refresh_G1h(cdlgb_ctx* c) {
 
 float* cur_X(cdlgb_ctx* c) { return c->Xb[c->xcur]; }
 
+// blocks of kBlock threads that take `per` of n items at a time, up to `most`: beyond the
+// work there is, a block only adds to the partial sums
+int blocks_for(size_t n, int per, int most) {
+    return (int)std::max<size_t>(1, std::min<size_t>((n + (size_t)per * kBlock - 1) / ((size_t)per * kBlock), most));
+}
+// last_block's counter: zeroed at allocation, zero again after every launch
+unsigned* block_counter(cdlgb_ctx* c) { return reinterpret_cast<unsigned*>(c->dscalar + 7); }
+
 }  // namespace
 
 // ============================================================================ API-level
@@ -745,8 +763,6 @@ int admm_alloc(cdlgb_ctx* c) {
         if (spec) {
             ST_TRY(A((void**)&c->g1h, nmf * 8));
             ST_TRY(A((void**)&c->Dg, (size_t)c->M * c->F * 8));
-            ST_TRY(A((void**)&c->G3h, (size_t)c->M * c->F * 8));
-            ST_TRY(A((void**)&c->sumspec, (size_t)3 * c->M * c->F * 8));
         }
     }
     c->dh_valid = 0;
@@ -755,10 +771,13 @@ int admm_alloc(cdlgb_ctx* c) {
     ST_TRY(A((void**)&c->Y1, LN * 4));
     ST_TRY(A((void**)&c->y1, LN * 4));
     ST_TRY(A((void**)&c->DX, LN * 4));
-    ST_TRY(A((void**)&c->Td, LN * 4));
+    // with the spectral D-step, the rows of G3, its spectrum, the sums' spectra and the sums
+    // lie behind the N rows that are transformed the same way (admm_dict_update)
+    const size_t MF = (size_t)c->M * c->F, NF = (size_t)c->N * c->F;
+    ST_TRY(A((void**)&c->Td, (LN + (spec ? 3 * LM : 0)) * 4));
     ST_TRY(A((void**)&c->G2, LN * 4));
     ST_TRY(A((void**)&c->g2, LN * 4));
-    ST_TRY(A((void**)&c->sU, LN * 4));
+    ST_TRY(A((void**)&c->sU, (LN + (spec ? LM : 0)) * 4));
     ST_TRY(A((void**)&c->G1, LM * 4));
     ST_TRY(A((void**)&c->G3, LM * 4));
     ST_TRY(A((void**)&c->dsum, LM * 4));
@@ -766,8 +785,10 @@ int admm_alloc(cdlgb_ctx* c) {
     ST_TRY(A((void**)&c->vbar, LM * 4));
     ST_TRY(A((void**)&c->G1h, (size_t)c->M * c->F * 8));
     ST_TRY(A((void**)&c->Ah, (size_t)c->F * 4));
-    ST_TRY(A((void**)&c->sUh, (size_t)c->N * c->F * 8));
-    ST_TRY(A((void**)&c->sVh, (size_t)c->N * c->F * 8));
+    ST_TRY(A((void**)&c->sUh, (NF + (spec ? MF : 0)) * 8));
+    ST_TRY(A((void**)&c->sVh, (NF + (spec ? 3 * MF : 0)) * 8));
+    c->G3h = spec ? c->sUh + NF : nullptr;
+    c->sumspec = spec ? c->sVh + NF : nullptr;
     // cuFFT-path scratch for one chunk of sequences (init's DX, the D-step, and the
     // X-step when no fused kernel covers Lg)
     c->chunk = chunk_for(c->N, c->M, c->Lg);
@@ -786,10 +807,11 @@ int admm_alloc(cdlgb_ctx* c) {
     ST_TRY(A((void**)&c->sBh, cSp * 8));
     ST_TRY(A((void**)&c->sCh, cSp * 8));
     c->nchunk = std::max(1, std::min(64, c->N));
-    ST_TRY(A((void**)&c->part, (size_t)c->nchunk * 3 * LM * 4));
+    if (!spec) ST_TRY(A((void**)&c->part, (size_t)c->nchunk * 3 * LM * 4));
     c->nred = 152 * 4;
     ST_TRY(A((void**)&c->dred, (size_t)c->nred * 4 * sizeof(double)));
     ST_TRY(A((void**)&c->dscalar, 8 * sizeof(double)));
+    CU_TRY(c, cudaMemsetAsync(c->dscalar, 0, 8 * sizeof(double), c->stream));
     c->hscalar = host_scalars_get();
     c->hscalar_own = false;
     if (!c->hscalar) {
@@ -808,8 +830,9 @@ void admm_free(cdlgb_ctx* c) {
                     &c->dsum, &c->Dbest, &c->vbar, &c->Ah, &c->sA, &c->sB, &c->part};
     for (auto p : fl) { dev_free(c, *p); *p = nullptr; }
     float2** cl[] = {&c->G1h, &c->sUh, &c->sVh, &c->sAh, &c->sBh, &c->sCh, &c->Dhs,
-                     &c->g1h, &c->Dg, &c->G3h, &c->spart, &c->sumspec};
+                     &c->g1h, &c->Dg, &c->spart};
     for (auto p : cl) { dev_free(c, *p); *p = nullptr; }
+    c->G3h = c->sumspec = nullptr;
     dev_free(c, c->dred);
     dev_free(c, c->dscalar);
     if (c->hscalar) {
@@ -861,7 +884,7 @@ int admm_write_duals(cdlgb_ctx* c) {
 
 int admm_init(cdlgb_ctx* c, const float* X0, const float* D0, uint64_t seed) {
     cudaStream_t s = c->stream;
-    const int Lg = c->Lg, M = c->M, N = c->N, flen = 4 * c->p.filter_size;
+    const int Lg = c->Lg, M = c->M, flen = 4 * c->p.filter_size;
     const size_t LMN = c->LMN, LN = c->LN, LM = c->LM;
     c->xcur = 0;
     c->best_is_cur = 1;
@@ -1014,10 +1037,14 @@ int admm_dict_update(cdlgb_ctx* c, int iters) {
         cdlgb_phase_begin(c, PH_DSTEP);
         if (c->dspec) {
             // the state in the frequency domain: only Y3 is transformed (dspec.cu)
-            k_sub<<<grid_for(LN, kBlock), kBlock, 0, s>>>(c->G2, c->g2, c->sU, LN);
+            // with cuFFT's rows, G2 - g2 and G3 go in one transform, Td and the sums below come
+            // in one (the register transforms pair the rows of each on their own)
+            const bool joint = !row_plan(c);
+            float* sums = c->Td + LN;
+            k_sub<<<grid_for(LN + LM, kBlock), kBlock, 0, s>>>(c->G2, c->g2, c->sU, LN, c->G3, joint ? LM : 0);
             LAUNCH_CHECK(c, "k_sub");
-            ST_TRY(r2c(c, N, c->sU, c->sUh, 1));
-            ST_TRY(r2c(c, M, c->G3, c->G3h, M));
+            ST_TRY(r2c(c, joint ? N + M : N, c->sU, c->sUh, 1));
+            if (!joint) ST_TRY(r2c(c, M, c->G3, c->G3h, M));
             void* fw = fused_dfwd(c);
             int slot0 = 0;
             for (int n0 = 0; n0 < N; n0 += c->schunk) {
@@ -1044,19 +1071,19 @@ int admm_dict_update(cdlgb_ctx* c, int iters) {
             }
             c->spec_init = 0;
             if (c->res_on) ST_TRY(resid_d_from_spec_parts(c, slot0 * ((F + 31) / 32)));
-            ST_TRY(c2r(c, N, c->sVh, c->Td, 1));
+            // Td, and the three sums over n as k_dfinish's one chunk
+            ST_TRY(dspec_sums(c, c->G3h, c->sumspec));
+            ST_TRY(c2r(c, joint ? N + 3LL * M : N, c->sVh, c->Td, 1));
+            if (!joint) ST_TRY(c2r(c, 3LL * M, c->sumspec, sums, 3 * M));
             k_dg2<<<grid_for(LN, kBlock), kBlock, 0, s>>>(c->Td, c->g2, c->G2, c->S, Lg, c->L4,
                                                          c->gamma, LN, c->p.sigma);
             LAUNCH_CHECK(c, "k_dg2");
             if (c->res_on) ST_TRY(resid_td(c));
-            // the three sums over n, back in the time domain: part as one chunk
-            ST_TRY(dspec_sums(c, c->G3h, c->sumspec));
-            ST_TRY(c2r(c, 3LL * M, c->sumspec, c->part, 3 * M));
             c->time_stale = 1;
             c->time_init = 0;
             int flen = 4 * c->p.filter_size;
             if (c->res_on) ST_TRY(resid_save_G(c));
-            k_dfinish<<<(unsigned)((LM + 255) / 256), 256, 0, s>>>(c->part, c->vbar, c->G3, c->dsum,
+            k_dfinish<<<(unsigned)((LM + 255) / 256), 256, 0, s>>>(sums, c->vbar, c->G3, c->dsum,
                                                                    LM, Lg, flen, N, 1);
             LAUNCH_CHECK(c, "k_dfinish");
             k_dprox<<<(unsigned)((LM + 255) / 256), 256, 0, s>>>(c->vbar, c->G1, Lg, M, flen);
@@ -1067,7 +1094,7 @@ int admm_dict_update(cdlgb_ctx* c, int iters) {
             continue;
         }
         {
-            k_sub<<<grid_for(LN, kBlock), kBlock, 0, s>>>(c->G2, c->g2, c->sU, LN);
+            k_sub<<<grid_for(LN, kBlock), kBlock, 0, s>>>(c->G2, c->g2, c->sU, LN, nullptr, 0);
             LAUNCH_CHECK(c, "k_sub");
             ST_TRY(r2c(c, N, c->sU, c->sUh, 1));
             void* fw = c->fused && c->Dhs ? fused_dfwd(c) : nullptr;
@@ -1128,11 +1155,10 @@ int admm_dict_update(cdlgb_ctx* c, int iters) {
     return CDLGB_OK;
 }
 
-// objective into c->dscalar[0] (device), no host sync
+// objective into the pinned c->hscalar[0], no host sync
 static int objective_async(cdlgb_ctx* c) {
     cudaStream_t s = c->stream;
     int nb1 = 152 * 2;
-    const int nb2 = kFitBlocks;
     const double* pa = c->dred;
     const double* fp = nullptr;
     int nf = 0;
@@ -1149,20 +1175,17 @@ static int objective_async(cdlgb_ctx* c) {
         k_abssum<<<nb1, kBlock, 0, s>>>((const float4*)cur_X(c), c->LMN / 4, c->dred);
         LAUNCH_CHECK(c, "k_abssum");
     }
-    k_fit<<<nb2, kBlock, 0, s>>>((const float4*)c->DX, (const float4*)c->S, c->Lg / 4, c->L4 / 4, c->gamma / 4,
-                                 (size_t)c->N * (c->L4 / 4), c->dred + 152 * 2);
+    const size_t n4 = (size_t)c->N * (c->L4 / 4);
+    k_fit<<<blocks_for(n4, 4, kFitBlocks), kBlock, 0, s>>>(
+        (const float4*)c->DX, (const float4*)c->S, c->Lg / 4, c->L4 / 4, c->gamma / 4, n4, c->dred + 152 * 2, pa, nb1,
+        (double)c->p.lambda, block_counter(c), c->hscalar);
     LAUNCH_CHECK(c, "k_fit");
-    k_obj_final<<<1, kBlock, 0, s>>>(pa, nb1, c->dred + 152 * 2, nb2, (double)c->p.lambda,
-                                     c->dscalar);
-    LAUNCH_CHECK(c, "k_obj_final");
     return CDLGB_OK;
 }
 
 int admm_objective(cdlgb_ctx* c, double* obj) {
     cdlgb_phase_begin(c, PH_OBJ);
     ST_TRY(objective_async(c));
-    CU_TRY(c, cudaMemcpyAsync(c->hscalar, c->dscalar, sizeof(double), cudaMemcpyDeviceToHost,
-                              c->stream));
     cdlgb_phase_end(c, PH_OBJ);
     CU_TRY(c, cudaStreamSynchronize(c->stream));
     *obj = c->hscalar[0];
@@ -1189,16 +1212,13 @@ int admm_update_best(cdlgb_ctx* c, double* obj, int* improved) {
 int admm_code_threshold(cdlgb_ctx* c, double* thr) {
     cudaStream_t s = c->stream;
     const float* Xbest = c->best_is_cur ? c->Xb[c->xcur] : c->Xb[1 - c->xcur];
-    const int nb = kPosBlocks;
-    k_pos_stats<false><<<nb, kBlock, 0, s>>>((const float4*)Xbest, c->LMN / 4, nullptr, c->dred);
+    const int nb = blocks_for(c->LMN / 4, 8, kPosBlocks);
+    k_pos_stats<false><<<nb, kBlock, 0, s>>>((const float4*)Xbest, c->LMN / 4, c->dred, c->dscalar, block_counter(c),
+                                             nullptr);
     LAUNCH_CHECK(c, "k_pos_stats");
-    k_pos_final<<<1, kBlock, 0, s>>>(c->dred, nb, c->dscalar, 0);
-    LAUNCH_CHECK(c, "k_pos_final");
-    k_pos_stats<true><<<nb, kBlock, 0, s>>>((const float4*)Xbest, c->LMN / 4, c->dscalar + 1, c->dred);
+    k_pos_stats<true><<<nb, kBlock, 0, s>>>((const float4*)Xbest, c->LMN / 4, c->dred, c->dscalar, block_counter(c),
+                                            c->hscalar + 2);
     LAUNCH_CHECK(c, "k_pos_stats");
-    k_pos_final<<<1, kBlock, 0, s>>>(c->dred, nb, c->dscalar, 1);
-    LAUNCH_CHECK(c, "k_pos_final");
-    CU_TRY(c, cudaMemcpyAsync(c->hscalar, c->dscalar, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
     CU_TRY(c, cudaStreamSynchronize(s));
     *thr = c->hscalar[2] * (double)c->p.std_threshold_multiplier;
     return CDLGB_OK;

@@ -102,7 +102,7 @@ __global__ void k_check_onehot(const float4* __restrict__ S, size_t n4, int* __r
 }
 
 static int check_onehot(cdlgb_ctx* c) {
-    int* flag = (int*)c->dscalar;      // 8 doubles of device scratch, first int used here
+    int* flag = (int*)c->dscalar;      // 8 doubles of device scratch, its first int used here
     CU_TRY(c, cudaMemsetAsync(flag, 0, sizeof(int), c->stream));
     size_t n4 = (size_t)c->L4 * c->N / 4;
     k_check_onehot<<<grid_for(n4, 256), 256, 0, c->stream>>>((const float4*)c->S, n4, flag);

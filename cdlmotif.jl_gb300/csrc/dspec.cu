@@ -420,11 +420,12 @@ __global__ void __launch_bounds__(kBins * kWarps, 1) k_dspec_wide(SArgs A) {
 
 // The three sums' spectra, scaled by 1/Lg so that the unnormalised inverse transform
 // gives the time-domain sums: out[0] = sum (d + g1), out[2] = sum d (over the slots, in
-// double), out[1] = sum (d + g3) = out[0] - N Dg (Dg after this D-step's update).  Four
+// double), out[1] = sum (d + g3) = out[0] - N Dg after this D-step's Dg += G3-hat - G1-hat
+// (the change of g1 - g3, train.jl:70, 72; the solves have used the old one).  Four
 // threads per output take the slots j = t mod 4 in order; the four partials are added in
 // a fixed order.
-__global__ void k_dspec_sum(const float2* __restrict__ part, const float2* __restrict__ Dg,
-                            float2* __restrict__ out, size_t mf, int slots, int N, double inv_lg) {
+__global__ void k_dspec_sum(const float2* __restrict__ part, float2* __restrict__ Dg,
+                            const float2* __restrict__ G1h, const float2* __restrict__ G3h, float2* __restrict__ out, size_t mf, int slots, int N, double inv_lg) {
     const size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     const size_t i = g >> 2;                                // 0 .. 2 mf - 1
     const int t = (int)(g & 3);
@@ -442,20 +443,13 @@ __global__ void k_dspec_sum(const float2* __restrict__ part, const float2* __res
     if (t != 0 || i >= 2 * mf) return;
     if (i < mf) {
         out[i] = make_float2((float)(re * inv_lg), (float)(im * inv_lg));
-        const float2 dg = Dg[i];
+        const float2 dg = cadd2(Dg[i], csub2(G3h[i], G1h[i]));
+        Dg[i] = dg;
         out[mf + i] = make_float2((float)((re - (double)N * dg.x) * inv_lg),
                                   (float)((im - (double)N * dg.y) * inv_lg));
     } else {
         out[mf + i] = make_float2((float)(re * inv_lg), (float)(im * inv_lg));
     }
-}
-
-// Dg += G3-hat - G1-hat (the change of g1 - g3 in one D-step, train.jl:70, 72)
-__global__ void k_dg_update(float2* __restrict__ Dg, const float2* __restrict__ G1h,
-                            const float2* __restrict__ G3h, size_t mf) {
-    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (i >= mf) return;
-    Dg[i] = cadd2(Dg[i], csub2(G3h[i], G1h[i]));
 }
 
 // dst = a - plane, the plane broadcast over n (g3-hat = g1-hat - Dg)
@@ -545,10 +539,8 @@ int dspec_launch(cdlgb_ctx* c, const float2* Yh, const float2* G3h, int c0, int 
 // the Dg update (after every chunk has used the old Dg) and the three sums: out (3, M, F)
 int dspec_sums(cdlgb_ctx* c, const float2* G3h, float2* out) {
     const size_t mf = (size_t)c->M * c->F;
-    k_dg_update<<<(unsigned)((mf + 255) / 256), 256, 0, c->stream>>>(c->Dg, c->G1h, G3h, mf);
-    LAUNCH_CHECK(c, "k_dg_update");
     k_dspec_sum<<<(unsigned)((4 * 2 * mf + 255) / 256), 256, 0, c->stream>>>(
-        c->spart, c->Dg, out, mf, c->dslots, c->N, 1.0 / (double)c->Lg);
+        c->spart, c->Dg, c->G1h, G3h, out, mf, c->dslots, c->N, 1.0 / (double)c->Lg);
     LAUNCH_CHECK(c, "k_dspec_sum");
     return CDLGB_OK;
 }
