@@ -275,16 +275,18 @@ __device__ __forceinline__ void xprep1(float x, float a, float b, float lam, boo
 
 // xprep1 for the two filters of a slot at once (packed FP32x2: the same operations
 // on both halves, so the same bits); y2 and y3 are updated in place, V returned
-__device__ __forceinline__ float2 xprep2(float2 x, float2& y2, float2& y3, float lam, bool keep) {
-    const float2 t = cadd(x, y2);
+// ... from t = X + y2 and u = X + y3, which is all that V and the new duals depend on
+__device__ __forceinline__ float2 xsplit2(float2 t, float2 u, float2& y2, float2& y3, float lam, bool keep) {
     const float2 c = f2(fminf(fmaxf(t.x, -lam), lam), fminf(fmaxf(t.y, -lam), lam));
     const float2 Y2 = csub(t, c);
     const float2 na = csub(t, Y2);
-    const float2 u = cadd(x, y3);
     const float2 w = csub(Y2, na);
     y2 = na;
     y3 = keep ? f2(0.f, 0.f) : u;
     return keep ? cadd(w, u) : csub(w, u);
+}
+__device__ __forceinline__ float2 xprep2(float2 x, float2& y2, float2& y3, float lam, bool keep) {
+    return xsplit2(cadd(x, y2), cadd(x, y3), y2, y3, lam, keep);
 }
 
 

@@ -11,10 +11,14 @@
 // An X-step has two parts:
 //   codes   a CTA takes B pairs of filters of one sequence: X from the previous step's V
 //           and W, then shrink!, projectionX! and the dual updates (csc_kernels.jl:53-82,
-//           train.jl:12-14) give this step's V, which is stored in X's place and, through
-//           shared memory, convolved with the taps into the CTA's part of P;
+//           train.jl:12-14) give this step's V, which goes through shared memory and is
+//           convolved with the taps into the CTA's part of P;
 //   solve   a CTA takes one sequence: P, the transforms, W, DX, Y1 (update_Y1!,
 //           csc_kernels.jl:86-95), y1 and U.
+// Between the steps a code is kept as t = X + y2 and u = X + y3, from which V and both duals
+// follow by the operations that define them (xsplit2: the same bits): two arrays read and
+// written per X-step instead of V, y2 and y3 (a code update of 15 X-steps 3.60 -> 3.43 ms at
+// 5000 sequences, L = 200, 10 filters of 4 bases, 8.18 -> 7.81 at 500, 1000, 32, 16).
 // Each is a launch over all sequences (k_xc_codes, k_xc_solve), started early with
 // griddepcontrol; where one CTA holds all filters of a sequence and all sequences are
 // resident at once, one launch runs all X-steps instead (k_xc_all).
@@ -51,9 +55,9 @@ __device__ __forceinline__ float2 unpack(f32x2 a) {
 
 struct Args {
     const float* Xin;       // X
-    float* V;               // V between the steps, X after the last
-    float* y2;
-    float* y3;
+    float* V;               // t = X + y2 between the steps, X after the last
+    float* y2;              // read by the first, written after the last
+    float* y3;              // u = X + y3 between the steps
     float* Y1;
     float* y1;
     float* DX;
@@ -272,7 +276,8 @@ __device__ __forceinline__ void solve(const Args& A, float2* buf, size_t c, size
     }
 }
 
-// FIRST: V from X; MID: X from the previous V and W, then V; LAST: X only.
+// FIRST: t, u and V from X and the duals; MID: X from the previous V and W, then t, u and V;
+// LAST: X and the duals.
 // A thread owns 16 consecutive rows of a pair of filters, two packed floats per row: it
 // keeps 16 sums in registers and slides over the taps, one shared-memory load per 16
 // packed FMAs.  gs: [8 NB][B] two taps of a pair; ws: [9 (nchunk + NB)] two values of W,
@@ -335,7 +340,7 @@ __device__ __forceinline__ float codes(const Args& A, const float4* gs, const fl
         int pp = 0, k4 = lane;
         for (int e = lane; e < groups; e += 64) {
             // two groups of four rows in flight
-            float4 xa[2], xb[2], aa[2], ab[2], ba[2], bb[2];
+            float4 xa[2], xb[2], aa[2], ab[2], ba[2], bb[2];       // X (t), y2, y3 (u) of both filters
             int pu[2], ku[2];
             size_t ra[2];
 #pragma unroll
@@ -351,11 +356,13 @@ __device__ __forceinline__ float codes(const Args& A, const float4* gs, const fl
                 xb[u] = two ? *reinterpret_cast<const float4*>(src + Lg) : z4;
                 if (MODE == FIRST && A.zero) {
                     aa[u] = ab[u] = ba[u] = bb[u] = z4;
-                } else if (MODE != LAST) {
-                    aa[u] = on ? *reinterpret_cast<const float4*>(A.y2 + ra[u]) : z4;
+                } else {
                     ba[u] = on ? *reinterpret_cast<const float4*>(A.y3 + ra[u]) : z4;
-                    ab[u] = two ? *reinterpret_cast<const float4*>(A.y2 + ra[u] + Lg) : z4;
                     bb[u] = two ? *reinterpret_cast<const float4*>(A.y3 + ra[u] + Lg) : z4;
+                    if (MODE == FIRST) {
+                        aa[u] = on ? *reinterpret_cast<const float4*>(A.y2 + ra[u]) : z4;
+                        ab[u] = two ? *reinterpret_cast<const float4*>(A.y2 + ra[u] + Lg) : z4;
+                    }
                 }
                 k4 += 32;
             }
@@ -365,28 +372,43 @@ __device__ __forceinline__ float codes(const Args& A, const float4* gs, const fl
                 const bool two = 2 * pu[u] + 1 < Mr;
                 const int l = R * q0 + 4 * ku[u];
                 float2 x[4] = {f2(xa[u].x, xb[u].x), f2(xa[u].y, xb[u].y), f2(xa[u].z, xb[u].z), f2(xa[u].w, xb[u].w)};
+                float2 a3[4] = {f2(ba[u].x, bb[u].x), f2(ba[u].y, bb[u].y), f2(ba[u].z, bb[u].z), f2(ba[u].w, bb[u].w)};
+                float2 a2[4];
+                if (MODE == FIRST) {
+                    a2[0] = f2(aa[u].x, ab[u].x);
+                    a2[1] = f2(aa[u].y, ab[u].y);
+                    a2[2] = f2(aa[u].z, ab[u].z);
+                    a2[3] = f2(aa[u].w, ab[u].w);
+                }
                 float2* vq = Vs + pu[u] * A.pitch + 17 * (q0 + (ku[u] >> 2) + NB) + 4 * (ku[u] & 3);
                 if (MODE != FIRST) {
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        x[k] = cadd(x[k], vq[k]);
+                        const float2 v = xsplit2(x[k], a3[k], a2[k], a3[k], lam, k == 0);
+                        x[k] = cadd(v, vq[k]);
                         x[k] = f2(x[k].x * ik, x[k].y * ik);
                     }
                 }
                 float* dst = A.V + ra[u];
                 if (MODE == LAST) {
                     *reinterpret_cast<float4*>(dst) = make_float4(x[0].x, x[1].x, x[2].x, x[3].x);
-                    if (two) *reinterpret_cast<float4*>(dst + Lg) = make_float4(x[0].y, x[1].y, x[2].y, x[3].y);
+                    *reinterpret_cast<float4*>(A.y2 + ra[u]) = make_float4(a2[0].x, a2[1].x, a2[2].x, a2[3].x);
+                    *reinterpret_cast<float4*>(A.y3 + ra[u]) = make_float4(0.f, a3[1].x, a3[2].x, a3[3].x);
+                    if (two) {
+                        *reinterpret_cast<float4*>(dst + Lg) = make_float4(x[0].y, x[1].y, x[2].y, x[3].y);
+                        *reinterpret_cast<float4*>(A.y2 + ra[u] + Lg) = make_float4(a2[0].y, a2[1].y, a2[2].y, a2[3].y);
+                        *reinterpret_cast<float4*>(A.y3 + ra[u] + Lg) = make_float4(0.f, a3[1].y, a3[2].y, a3[3].y);
+                    }
 #pragma unroll
                     for (int k = 0; k < 4; ++k) absacc += fabsf(x[k].x) + fabsf(x[k].y);
                     continue;
                 }
-                float2 a2[4] = {f2(aa[u].x, ab[u].x), f2(aa[u].y, ab[u].y), f2(aa[u].z, ab[u].z), f2(aa[u].w, ab[u].w)};
-                float2 a3[4] = {f2(ba[u].x, bb[u].x), f2(ba[u].y, bb[u].y), f2(ba[u].z, bb[u].z), f2(ba[u].w, bb[u].w)};
-                float2 v[4];
+                float2 v[4], w[4];                                   // V; u (x becomes t)
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    v[k] = xprep2(x[k], a2[k], a3[k], lam, k == 0);
+                    w[k] = cadd(x[k], a3[k]);
+                    x[k] = cadd(x[k], a2[k]);
+                    v[k] = xsplit2(x[k], w[k], a2[k], a3[k], lam, k == 0);
                     vq[k] = v[k];
                 }
                 if (l + 3 >= Lg - TP) {                              // again before the first row
@@ -396,13 +418,11 @@ __device__ __forceinline__ float codes(const Args& A, const float4* gs, const fl
                         if (at >= 0) Vs[pu[u] * A.pitch + fp(at)] = v[k];
                     }
                 }
-                *reinterpret_cast<float4*>(dst) = make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
-                *reinterpret_cast<float4*>(A.y2 + ra[u]) = make_float4(a2[0].x, a2[1].x, a2[2].x, a2[3].x);
-                *reinterpret_cast<float4*>(A.y3 + ra[u]) = make_float4(0.f, a3[1].x, a3[2].x, a3[3].x);
+                *reinterpret_cast<float4*>(dst) = make_float4(x[0].x, x[1].x, x[2].x, x[3].x);
+                *reinterpret_cast<float4*>(A.y3 + ra[u]) = make_float4(w[0].x, w[1].x, w[2].x, w[3].x);
                 if (two) {
-                    *reinterpret_cast<float4*>(dst + Lg) = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
-                    *reinterpret_cast<float4*>(A.y2 + ra[u] + Lg) = make_float4(a2[0].y, a2[1].y, a2[2].y, a2[3].y);
-                    *reinterpret_cast<float4*>(A.y3 + ra[u] + Lg) = make_float4(0.f, a3[1].y, a3[2].y, a3[3].y);
+                    *reinterpret_cast<float4*>(dst + Lg) = make_float4(x[0].y, x[1].y, x[2].y, x[3].y);
+                    *reinterpret_cast<float4*>(A.y3 + ra[u] + Lg) = make_float4(w[0].y, w[1].y, w[2].y, w[3].y);
                 }
             }
         }
@@ -552,8 +572,8 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_xc_codes(const __grid_consta
     // this CTA's rows towards L2 while it convolves (hints; a row is a multiple of 16 bytes)
     if (MODE != FIRST && threadIdx.x >= blockDim.x - 32) {
         const size_t r0 = (n * A.M + m0) * A.Lg;
-        for (int k = threadIdx.x & 31; k < (MODE == LAST ? 1 : 3) * Mr; k += 32) {
-            const float* a = (k < Mr ? A.V : k < 2 * Mr ? A.y2 : A.y3) + r0 + (size_t)(k % Mr) * A.Lg;
+        for (int k = threadIdx.x & 31; k < 2 * Mr; k += 32) {
+            const float* a = (k < Mr ? A.V : A.y3) + r0 + (size_t)(k % Mr) * A.Lg;
             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" :: "l"(a), "r"(4 * A.Lg) : "memory");
         }
     }
