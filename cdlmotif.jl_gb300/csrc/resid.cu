@@ -16,6 +16,8 @@
 // deterministic for a given size and device.
 #include "cdlgb_internal.h"
 
+#include <algorithm>
+
 namespace {
 
 constexpr int kRB = 256;       // threads per block of the partial-sum kernels
@@ -133,31 +135,20 @@ __global__ void k_res_sum(const double* __restrict__ part, int nb, int nv, doubl
     if (lane == 0) out[map.idx[k]] = scale * t;
 }
 
-// the D-step's dual residual: N sum (G1 - G1_old)^2, N sum (G3 - G3_old)^2 and
-// N (sum G1^2 + sum G3^2); one block, fixed order
+// the D-step's dual residual: sums of (G1 - G1_old)^2, (G3 - G3_old)^2 and G1^2 + G3^2 per
+// block (k_res_sum multiplies by N; in one block they held a D-step of 25 filters of 620 rows
+// for 53 of its 311 us)
 __global__ void k_gdual(const float* __restrict__ G1, const float* __restrict__ G3,
-                        const float* __restrict__ Gprev, size_t lm, int N, double* __restrict__ out) {
+                        const float* __restrict__ Gprev, size_t lm, double* __restrict__ part) {
     double v[3] = {0.0, 0.0, 0.0};
-    for (size_t i = threadIdx.x; i < lm; i += blockDim.x) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < lm; i += (size_t)gridDim.x * blockDim.x) {
         const float a = G1[i], b = G3[i];
         const double e1 = (double)a - (double)Gprev[i], e3 = (double)b - (double)Gprev[lm + i];
         v[0] += e1 * e1;
         v[1] += e3 * e3;
         v[2] += (double)a * a + (double)b * b;
     }
-    __shared__ double sh[3][32];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        v[k] = warp_sum_d(v[k]);
-        if (lane == 0) sh[k][w] = v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x < 3) {
-        double t = 0.0;
-        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += sh[threadIdx.x][i];
-        out[RESIDUAL_DUAL_G1 + threadIdx.x] = (double)N * t;
-    }
+    block_partials<3>(v, part);
 }
 
 // the stopping test's relative residuals and their maximum, from the raw sums
@@ -251,7 +242,11 @@ int resid_save_G(cdlgb_ctx* c) {
 
 // the dual residual after the projections, then the relative residuals
 int resid_dual_and_finish(cdlgb_ctx* c) {
-    k_gdual<<<1, 512, 0, c->stream>>>(c->G1, c->G3, c->Gprev, c->LM, c->N, c->dres);
+    const int nb = (int)std::min<size_t>((c->LM + kRB - 1) / kRB, 152);
+    k_gdual<<<nb, kRB, 0, c->stream>>>(c->G1, c->G3, c->Gprev, c->LM, c->rpart);
     LAUNCH_CHECK(c, "k_gdual");
+    ResMap m = {{RESIDUAL_DUAL_G1, RESIDUAL_DUAL_G3, RESIDUAL_G_NORM, 0, 0}};
+    k_res_sum<<<1, 3 * 32, 0, c->stream>>>(c->rpart, nb, 3, (double)c->N, m, c->dres);
+    LAUNCH_CHECK(c, "k_res_sum");
     return resid_finish(c);
 }
