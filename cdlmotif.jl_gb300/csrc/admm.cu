@@ -562,7 +562,7 @@ __global__ void __launch_bounds__(256) k_pos_stats(const float4* __restrict__ X,
     }
 }
 
-// host-side seeded normal (used for D0 when none is given)
+// host-side seeded uniform (the simplex draw of D0)
 double host_uniform(uint64_t seed, uint64_t i) {
     uint64_t h = splitmix64(seed * 0x9E3779B97F4A7C15ull ^ (i + 0x51ull));
     return ((double)(h >> 11) + 0.5) * (1.0 / 9007199254740992.0);

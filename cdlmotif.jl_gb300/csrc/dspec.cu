@@ -530,7 +530,8 @@ int dspec_launch(cdlgb_ctx* c, const float2* Yh, const float2* G3h, int c0, int 
                       (size_t)5 * kBins * sizeof(float);
     auto k = c->res_on ? (c->spec_init ? k_dspec_wide<true, true> : k_dspec_wide<true, false>)
                        : (c->spec_init ? k_dspec_wide<false, true> : k_dspec_wide<false, false>);
-    CU_TRY(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    // process-wide per kernel: the same cap for every context (M = 128 takes 107 KB)
+    CU_TRY(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
     k<<<g, kBins * kWarps, sm, c->stream>>>(a);
     LAUNCH_CHECK(c, "k_dspec_wide");
     return CDLGB_OK;

@@ -271,13 +271,14 @@ int init_x(cdlgb_ctx* c, float* X, bool draw, uint64_t seed, double* out, int* n
     a.pitch = (a.RA + Hp) / 8 * 12;
     // two rows of filters per part and per warp, in about a third of an SM's shared memory
     const int unit = std::max(a.ms, kWarps);
-    const size_t room = 72 * 1024;
+    constexpr size_t room = 72 * 1024;
     a.MG = (int)std::min<size_t>((size_t)2 * unit, std::max<size_t>(1, room / ((size_t)a.pitch * 4)));
     a.MG = std::min(a.MG, a.M);
     const size_t smem = std::max((size_t)a.MG * a.pitch * 4, (size_t)a.ms * a.nq * 9 * 16);
     auto k = draw ? k_init_x<true> : k_init_x<false>;
     int per_sm = 0;
-    CU_TRY(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // process-wide per kernel: the same cap for every context (smem is at most room)
+    CU_TRY(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
     CU_TRY(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kNT, smem));
     const size_t items = (size_t)a.N * a.nr;
     const int grid = (int)std::min<size_t>({items, (size_t)std::max(1, per_sm) * std::max(1, c->nsm), (size_t)kPart});

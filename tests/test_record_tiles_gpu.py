@@ -49,3 +49,26 @@ def test_topology_and_pairs_against_oracle(pkg, built_lib, N, L, M, sizes, densi
     finally:
         for c in ctxs:
             c.close()
+
+
+@pytest.mark.parametrize("longest", [5, 384, 768])
+def test_pair_pfms_with_room_for_long_spans(pkg, built_lib, longest):
+    """The span limit sets the shared memory of the pair sums (up to the 48 KB of float64 that
+    the last pass takes), not their values."""
+    N, L, M = 300, 60, 4
+    rng = np.random.default_rng(2)
+    S = pkg.synth.onehot(rng.integers(0, 4, (N, L)).astype(np.uint8))
+    with pkg.CDL(pkg.CDLSetup(M=M, filter_size=5)) as c, pkg.ActivationRecord(N, L, M, T=2) as ar:
+        c.load_data(S)
+        X = np.zeros((N, M, c.Lg), np.float32)
+        for t in (1, 2):                              # pairs are between trainings
+            X[:, :, c.gamma:c.gamma + 4 * L:4] = np.where(rng.random((N, M, L)) < 0.1, rng.uniform(1, 3, (N, M, L)), 0)
+            c.init_state(X0=X)
+            pkg.record_training_result(c, 0.5, ar, t, 5)
+        over = pkg.get_spatial_info(ar)[0]
+        thr = 0                                       # every pair that occurs
+        pairs, spans, pfms = pkg.get_pair_pfms(ar, c, over, thr, 5)
+        wide = pkg.get_pair_pfms(ar, c, over, thr, longest)
+    assert np.array_equal(pairs, wide[0]) and np.array_equal(spans, wide[1]) and len(pairs) > 0
+    for a, b in zip(pfms, wide[2]):
+        assert np.array_equal(a, b)
