@@ -425,7 +425,7 @@ constexpr int kLutSegs = 104;                             // KB of tables per CT
 
 struct LutArgs {
     const float* data;
-    const float* pwms;      // (K, 4, maxlen) col-major
+    const float* pwms;      // (K, 4, columns) col-major
     const int32_t* lens;
     const float* thresh;
     const int32_t* limit;   // [K] best approximations (+ 32768) from here on may hit
@@ -433,7 +433,7 @@ struct LutArgs {
     int32_t* pos;
     float* score;
     uint8_t* comp;
-    int K, KG, maxlen, L, N, words;                       // words: 32-position words of a sequence
+    int K, KG, widest, L, N, words;                       // widest: columns; words: 32-position words of a sequence
 };
 
 // the larger of each 16-bit half
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(32 * kLutWarps, 2) k_scan_lut(const __grid_con
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned full = 0xffffffffu;
     // the motifs, [motif][column][base], behind the tables and the warps' planes
-    const int kl = 4 * A.maxlen;
+    const int kl = 4 * A.widest;
     int segs = 0;
     for (int k = k0; k < k1; ++k) segs += (A.lens[k] + 3) / 4;
     unsigned* planes = reinterpret_cast<unsigned*>(lut + 256 * segs) + warp * 4 * (words + 1);   // [4][words + 1]
@@ -706,13 +706,15 @@ int check_pwm_args(cdlgb_ctx* c, const float* pwms, const int32_t* lens, const f
 
 // The filtered scans take motifs of at most 32 columns and sequences of at most 4096 bases;
 // the forward scan's threshold is not negative (below zero its first maximum can be a
-// window that is no hit).  Fills the motifs' scales and limits (as floats' bits) and the
-// motifs per CTA.
+// window that is no hit).  Fills the motifs' scales and limits (as floats' bits), the
+// motifs per CTA and the widest motif's columns: the array may be wider than any of them
+// (zero padding up to maxlen), and the tables go by the motifs alone.
 bool lut_ok(const cdlgb_ctx* c, const float* pwms, const int32_t* lens, const float* thresh, int K, int maxlen,
-            bool both, std::vector<float>& meta, int* KG) {
+            bool both, std::vector<float>& meta, int* KG, int* widest) {
     if (maxlen > 32 || c->L4 / 4 > 4096 || !sparse_ok(c, pwms, lens, K, maxlen)) return false;
     meta.resize(2 * (size_t)K);
     int segs = 0, most = 1;
+    *widest = 1;
     for (int k = 0; k < K; ++k) {
         if (!both && !(thresh[k] >= 0.f)) return false;
         double S = 0.0;
@@ -732,7 +734,8 @@ bool lut_ok(const cdlgb_ctx* c, const float* pwms, const int32_t* lens, const fl
                             : at > 65536.0 ? 65536 : at < 1.0 ? 1 : (int32_t)at;
         memcpy(&meta[K + k], &limit, 4);
         segs += ns;
-        most = ns > most ? ns : most;
+        most = std::max(most, ns);
+        *widest = std::max(*widest, (int)lens[k]);
     }
     const int parts = (segs + kLutSegs - 1) / kLutSegs;
     *KG = std::min((K + parts - 1) / parts, kLutSegs / most);
@@ -753,17 +756,19 @@ int upload_pwms(cdlgb_ctx* c, const float* pwms, const int32_t* lens, const floa
     return CDLGB_OK;
 }
 
-// the filtered scan of one or both strands; dmeta: 2 K floats of device scratch
+// The filtered scan of one or both strands; dmeta: 2 K floats of device scratch.  Shared
+// memory: KG ceil(widest / 4) <= kLutSegs KB of tables, at most 33 KB of planes (4096
+// bases) and KG 16 widest <= 6.5 KB of motifs.
 template <bool BOTH>
-int launch_lut(cdlgb_ctx* c, const std::vector<float>& meta, int KG, int K, int maxlen, int32_t* dpos, float* dscore,
-               uint8_t* dcomp, float* dmeta) {
+int launch_lut(cdlgb_ctx* c, const std::vector<float>& meta, int KG, int widest, int K, int maxlen, int32_t* dpos,
+               float* dscore, uint8_t* dcomp, float* dmeta) {
     CU_TRY(c, cudaMemcpyAsync(dmeta, meta.data(), (size_t)K * 8, cudaMemcpyHostToDevice, c->stream));
     LutArgs a;
     a.data = scan_data(c); a.pwms = c->scan_f; a.lens = c->scan_i; a.thresh = c->scan_f + (size_t)K * 4 * maxlen;
     a.scale = dmeta; a.limit = reinterpret_cast<const int32_t*>(dmeta + K); a.pos = dpos; a.score = dscore; a.comp = dcomp;
-    a.K = K; a.KG = KG; a.maxlen = maxlen; a.L = c->L4 / 4; a.N = c->N; a.words = (a.L + 31) / 32;
-    const size_t shm = (size_t)KG * ((maxlen + 3) / 4) * 1024 + (size_t)kLutWarps * 16 * (a.words + 1) +
-                       (size_t)KG * 16 * maxlen;
+    a.K = K; a.KG = KG; a.widest = widest; a.L = c->L4 / 4; a.N = c->N; a.words = (a.L + 31) / 32;
+    const size_t shm = (size_t)KG * ((widest + 3) / 4) * 1024 + (size_t)kLutWarps * 16 * (a.words + 1) +
+                       (size_t)KG * 16 * widest;
     CU_TRY(c, cudaFuncSetAttribute(k_scan_lut<BOTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 150 * 1024));
     const int parts = (K + KG - 1) / KG;
     const int gx = std::max(1, std::min((c->N + kLutWarps - 1) / kLutWarps, 2 * 152 / parts));
@@ -789,9 +794,9 @@ int scan_fwd(cdlgb_ctx* c, const float* pwms, const int32_t* lens, const float* 
     const size_t shs = (size_t)K * 4 * maxlen * sizeof(float) + (size_t)K * (nts / 32) * sizeof(VI) +
                        (size_t)L;
     std::vector<float> meta;
-    int KG = 0;
-    if (lut_ok(c, pwms, lens, thresh, K, maxlen, false, meta, &KG)) {
-        ST_TRY(launch_lut<false>(c, meta, KG, K, maxlen, dpos, nullptr, nullptr,
+    int KG = 0, widest = 0;
+    if (lut_ok(c, pwms, lens, thresh, K, maxlen, false, meta, &KG, &widest)) {
+        ST_TRY(launch_lut<false>(c, meta, KG, widest, K, maxlen, dpos, nullptr, nullptr,
                                  c->scan_f + (size_t)K * 4 * maxlen + K + (size_t)K * N));
     } else if (nts <= 1024 && shs <= 64 * 1024 && sparse_ok(c, pwms, lens, K, maxlen)) {
         if (shs > 48 * 1024)
@@ -834,9 +839,9 @@ int scan_both(cdlgb_ctx* c, const float* pwms, const int32_t* lens, const float*
     const size_t shp = (size_t)K * 4 * maxlen * sizeof(float2) + (size_t)K * (nts / 32) * 2 * sizeof(VI) +
                        (size_t)4 * ((L + 31) / 32 + 2) * sizeof(uint32_t);
     std::vector<float> meta;
-    int KG = 0;
-    if (lut_ok(c, pwms, lens, thresh, K, maxlen, true, meta, &KG)) {
-        ST_TRY(launch_lut<true>(c, meta, KG, K, maxlen, dpos, dscore, c->scan_u, dscore + (size_t)K * N));
+    int KG = 0, widest = 0;
+    if (lut_ok(c, pwms, lens, thresh, K, maxlen, true, meta, &KG, &widest)) {
+        ST_TRY(launch_lut<true>(c, meta, KG, widest, K, maxlen, dpos, dscore, c->scan_u, dscore + (size_t)K * N));
     } else if (nts <= 1024 && maxlen <= 64 && shp <= 64 * 1024 && sparse_ok(c, pwms, lens, K, maxlen)) {
         if (shp > 48 * 1024)
             CU_TRY(c, cudaFuncSetAttribute(k_scan_both_sparse, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
