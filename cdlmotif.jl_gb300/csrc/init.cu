@@ -253,15 +253,16 @@ int init_x(cdlgb_ctx* c, float* X, bool draw, uint64_t seed, double* out, int* n
     a.DX = (float4*)c->DX; a.G2 = (float4*)c->G2; a.out = out; a.seed = seed;
     a.N = c->N; a.M = c->M; a.La = c->Lg / 4; a.W = c->p.filter_size;
     // A range per CTA: a thread per 8 values, times as many filters at a time as fill the
-    // threads; a whole sequence at best.  Cut where a sequence is longer than the CTA, where
-    // more than a sixth of the threads would have no work, or where the ranges are fewer than
-    // the CTAs that fit; not below 16 threads along the range, where the values that are
-    // drawn twice (up to W + 7 per range) begin to count.
+    // threads; a whole sequence at best.  Cut where a sequence is longer than the CTA or where
+    // more than a sixth of the threads would have no work; not below 16 threads along the
+    // range, where the values that are drawn twice (up to W + 7 per range) begin to count.
+    // The number of sequences has no say: the cut sets ms, and with it the order of the sums
+    // over the filters, and a sequence's bits must not depend on how many others there are.
     const int chunks = (a.La + kRows - 1) / kRows;
     auto used = [&](int nq) { return std::min(kNT / nq, a.M) * nq; };
     for (a.nr = (chunks + kNT - 1) / kNT;; ++a.nr) {
         const int nq = (chunks + a.nr - 1) / a.nr, next = (chunks + a.nr) / (a.nr + 1);
-        if (next < 16 || (used(nq) * 6 >= kNT * 5 && (long long)a.N * a.nr >= 3LL * c->nsm)) break;
+        if (next < 16 || used(nq) * 6 >= kNT * 5) break;
     }
     a.nq = (chunks + a.nr - 1) / a.nr;
     a.RA = a.nq * kRows;
