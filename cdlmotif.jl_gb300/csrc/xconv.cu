@@ -63,10 +63,10 @@ struct Args {
     float* DX;
     const float* S;
     const float* G1;
-    float* P;               // [cn][G][Lg] parts of sum_m g_m (*) v_m
+    float* P;               // [cn][G][Lg] parts of sum_m g_m (*) v_m, of PB pairs each
     float* W;               // [cn][Lg]
     float* U;               // [cn][Lg]
-    double* absx_part;      // [N][G] sum |X|
+    double* absx_part;      // [N][CTAs per sequence] sum |X|
     const float2* tw;       // per stage [radix - 1][s] exp(-2 pi i o q / m), s = m / radix
     const float2* wk;       // [n/2 + 1] exp(-pi i k / n)
     const ushort2* pos;     // [n/2 + 1] places of bins k and n - k after the forward stages
@@ -77,6 +77,7 @@ struct Args {
     float lam, rho, kc;
     int NB;                 // blocks of 16 taps (the last one filled up with zeros)
     int B, CG, nchunk;      // pairs per CTA, row blocks per warp, row blocks
+    int PB, PCG;            // pairs per part of P, row blocks per warp that forms one
     int pitch;              // places of V per pair in shared memory
     int n, nst;
     int radix[kMaxStages], twoff[kMaxStages];
@@ -430,33 +431,37 @@ __device__ __forceinline__ float codes(const Args& A, const float4* gs, const fl
     return absacc;
 }
 
-// This CTA's part of P = sum_m g_m (*) v_m, as in codes(); the pairs of a row block sit in
-// neighbouring lanes, so the sum over them is a few shuffles.
-__device__ __forceinline__ void convolve(const Args& A, const float4* gs, const float2* Vs, float* Pt, int Mr) {
+// This CTA's parts of P = sum_m g_m (*) v_m, as in codes(): one (k_xc_codes, which holds a
+// part's pairs), or with ALL the A.G of its sequence, part g from pair g A.PB on, so that
+// either way a part is the same sum in the same order and solve() adds the same parts.  A
+// part's pairs of a row block sit in neighbouring lanes: the sum over them is a few shuffles.
+template <bool ALL>
+__device__ __forceinline__ void convolve(const Args& A, const float4* gs, const float2* Vs, float* P, int Mr) {
     constexpr int R = kR;
-    const int NB = A.NB, Lg = A.Lg, B = A.B;
+    const int NB = A.NB, Lg = A.Lg, B = A.PB, CG = A.PCG, GB = ALL ? A.B : B;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const int p = lane % B, cl = lane / B;
-    const bool lane_on = cl < A.CG && 2 * p < Mr;
-    const ulonglong2* gp = reinterpret_cast<const ulonglong2*>(gs) + p;
     const int pg2 = B >= 16 ? 16 : B >= 8 ? 8 : B >= 4 ? 4 : B >= 2 ? 2 : 1;
-    for (int q0 = warp * A.CG; q0 < A.nchunk; q0 += nwarps * A.CG) {
-        const int q = q0 + cl;
+    const int passes = (A.nchunk + CG - 1) / CG;                      // over a part's row blocks
+    for (int it = warp; it < (ALL ? A.G : 1) * passes; it += nwarps) {
+        const int part = ALL ? it / passes : 0, pr = part * B + p;
+        const int q = (it - part * passes) * CG + cl;
+        const bool lane_on = cl < CG && 2 * pr < Mr;
         f32x2 acc[R];
 #pragma unroll
         for (int i = 0; i < R; ++i) acc[i] = 0;
         if (lane_on && q < A.nchunk) {
-            const f32x2* v = reinterpret_cast<const f32x2*>(Vs + p * A.pitch + 17 * (q + NB));
+            const f32x2* v = reinterpret_cast<const f32x2*>(Vs + pr * A.pitch + 17 * (q + NB));
             f32x2 w[R];
 #pragma unroll
             for (int i = 0; i < R; ++i) w[i] = v[i];
-            const ulonglong2* gb = gp;
+            const ulonglong2* gb = reinterpret_cast<const ulonglong2*>(gs) + pr;
 #pragma unroll 1
-            for (int b = 0; b < NB; ++b, gb += 8 * B) {
+            for (int b = 0; b < NB; ++b, gb += 8 * GB) {
                 v -= 17;
 #pragma unroll
                 for (int j = 0; j < 16; j += 2) {
-                    const ulonglong2 gg = gb[(j >> 1) * B];
+                    const ulonglong2 gg = gb[(j >> 1) * GB];
 #pragma unroll
                     for (int i = 0; i < R; ++i) acc[i] = ffma2(gg.x, w[(i - j) & 15], acc[i]);
                     w[(-j - 1) & 15] = v[15 - j];
@@ -500,7 +505,8 @@ __device__ __forceinline__ void convolve(const Args& A, const float4* gs, const 
                 cnt = h;
             }
         }
-        if (cl < A.CG && p < pg2 && q < A.nchunk) {
+        if (cl < CG && p < pg2 && q < A.nchunk) {
+            float* Pt = P + (size_t)part * Lg;
             const int l = R * q + off;
 #pragma unroll
             for (int k = 0; k < R; ++k)
@@ -582,7 +588,7 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_xc_codes(const __grid_consta
     const float s = codes<MODE>(A, gs, ws, Vs, n, m0, Mr);
     __syncthreads();
     if (MODE == LAST) block_sum((double)s, A.absx_part + n * A.G + g);
-    else convolve(A, gs, Vs, A.P + (c * A.G + g) * A.Lg, Mr);
+    else convolve<false>(A, gs, Vs, A.P + (c * A.G + g) * A.Lg, Mr);
 }
 
 __global__ void __launch_bounds__(256) k_xc_solve(const __grid_constant__ Args A) {
@@ -617,7 +623,7 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_xc_all(const __grid_constant
             codes<MID>(A, gs, ws, Vs, n, 0, A.M);
         }
         __syncthreads();
-        convolve(A, gs, Vs, A.P + n * A.Lg, A.M);
+        convolve<true>(A, gs, Vs, A.P + n * A.G * A.Lg, A.M);
         __syncthreads();
         solve(A, Vs, n, n, it == 0, it == A.iters - 1);      // the transform in V's place
         __syncthreads();
@@ -746,6 +752,7 @@ struct Shape {
 
 struct XconvPlan {
     Shape s;
+    int G, PB, PCG;         // the parts of P: k_xc_codes's CTAs, in either form
     int n, nst, radix[kMaxStages], twoff[kMaxStages];
     int chunk, solve_threads;
     size_t solve_smem;
@@ -757,7 +764,7 @@ struct XconvPlan {
     double* cosL;           // cos(2 pi t / Lg), t < Lg
     double* cosN;           // cos(pi t / n), t < 2n
     double* h;              // [Lg/2 + 1] the solve's circular kernel
-    double* absx_part;      // [N][G]
+    double* absx_part;      // [N][s.G]
     int absx_n;
 };
 
@@ -836,27 +843,37 @@ void* xconv_plan_create(cdlgb_ctx* c, int slots, int* status) {
     P->solve_smem = (size_t)(n + n / 16 + 1) * sizeof(float2);
     P->solve_threads = n <= 512 ? 64 : n <= 1536 ? 128 : 256;
     const int T = 4 * c->p.filter_size;
-    // one CTA per sequence where that keeps every sequence resident (M <= 32)
-    int per_sm = 0;
-    if (c->M <= 32) {
-        P->s = shape_for(Lg, c->M, T, 16, n);
-        if (P->s.smem_all <= kSmemCta &&
-            (cudaFuncSetAttribute(k_xc_all, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCta) != cudaSuccess ||
-             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_xc_all, P->s.threads, P->s.smem_all) != cudaSuccess)) {
-            cudaGetLastError();
-            per_sm = 0;
-        }
-    }
-    P->all = c->N <= per_sm * c->nsm;
-    if (P->solve_smem > kSmemCta || (!P->all && !choose_shape(Lg, c->M, T, n, &P->s))) {
+    if (P->solve_smem > kSmemCta || !choose_shape(Lg, c->M, T, n, &P->s)) {
         delete P;
         return nullptr;
     }
-    const Shape& s = P->s;
+    P->G = P->s.G;
+    P->PB = P->s.B;
+    P->PCG = P->s.CG;
     // the parts of P lie in the cuFFT passes' scratch
-    P->chunk = (int)std::min<size_t>((size_t)c->chunk * c->M / s.G, c->N);
-    P->absx_n = c->N * s.G;
-    if (P->chunk < c->N) P->all = false;
+    P->chunk = (int)std::min<size_t>((size_t)c->chunk * c->M / P->G, c->N);
+    // one CTA per sequence where that keeps every sequence resident (M <= 32)
+    P->all = false;
+    if (c->M <= 32 && P->chunk == c->N) {
+        Shape a = shape_for(Lg, c->M, T, 16, n);
+        // as few warps as finish both passes (codes, parts of P) in the fewest rounds
+        const int codes_n = (a.nchunk + a.CG - 1) / a.CG, parts_n = P->G * ((a.nchunk + P->PCG - 1) / P->PCG);
+        const auto rounds = [&](int w) { return (codes_n + w - 1) / w + (parts_n + w - 1) / w; };
+        int warps = kMaxThreads / 32;
+        for (int w = warps; w >= 1; --w)
+            if (rounds(w) <= rounds(warps)) warps = w;
+        a.threads = 32 * warps;
+        int per_sm = 0;
+        if (a.smem_all <= kSmemCta &&
+            (cudaFuncSetAttribute(k_xc_all, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCta) != cudaSuccess ||
+             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_xc_all, a.threads, a.smem_all) != cudaSuccess)) {
+            cudaGetLastError();
+            per_sm = 0;
+        }
+        P->all = c->N <= per_sm * c->nsm;
+        if (P->all) P->s = a;
+    }
+    P->absx_n = c->N * P->s.G;
     Tables t = {};
     t.n = n;
     t.nst = P->nst;
@@ -935,7 +952,7 @@ int xconv_xsteps(cdlgb_ctx* c, void* p, const float* Xin, float* Xout, int iters
     a.absx_part = P->absx_part;
     a.tw = P->tw; a.wk = P->wk; a.pos = P->pos; a.Hsd = P->Hsd;
     a.M = c->M; a.Lg = c->Lg; a.L4 = c->L4; a.gamma = c->gamma; a.iters = iters;
-    a.T = 4 * c->p.filter_size; a.G = s.G;
+    a.T = 4 * c->p.filter_size; a.G = P->G; a.PB = P->PB; a.PCG = P->PCG;
     a.lam = c->p.lambda; a.rho = c->p.rho; a.kc = c->p.sherman_const_csc;
     a.NB = s.NB; a.B = s.B; a.CG = s.CG; a.nchunk = s.nchunk; a.pitch = s.pitch;
     a.n = P->n; a.nst = P->nst; a.zero = c->zero_duals;
