@@ -285,10 +285,11 @@ __device__ __forceinline__ void solve(const Args& A, float2* buf, size_t c, size
 // twice each, 16 values and a gap; Vs: [B][pitch], a row l of V at place l % 16 of row block
 // l / 16 + NB, 17 places of 8 bytes per block (the pitch has a residue modulo 16 for which
 // a warp's lanes, pair fastest, then block, spread over the banks); the NB blocks before
-// the first hold the last 16 NB rows again (the circular wrap).  Returns sum |X|.
+// the first hold the last 16 NB rows again (the circular wrap).  LAST returns sum |X|: four
+// rows of a filter in float32, as k_abssum adds them, and these in float64.
 enum { FIRST, MID, LAST };
 template <int MODE>
-__device__ __forceinline__ float codes(const Args& A, const float4* gs, const float4* ws, float2* Vs, size_t n, int m0,
+__device__ __forceinline__ double codes(const Args& A, const float4* gs, const float4* ws, float2* Vs, size_t n, int m0,
                                        int Mr) {
     constexpr int R = kR;
     const int NB = A.NB, TP = 16 * NB, Lg = A.Lg, B = A.B, M = A.M;
@@ -298,7 +299,7 @@ __device__ __forceinline__ float codes(const Args& A, const float4* gs, const fl
     const ulonglong2* gp = reinterpret_cast<const ulonglong2*>(gs) + p;
     const float lam = A.lam, ik = 1.f / A.kc;
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    float absacc = 0.f;
+    double absacc = 0.0;
     for (int q0 = warp * A.CG; q0 < A.nchunk; q0 += nwarps * A.CG) {
         // ---------------- sum_j g[j] W[l + j], left in V's place
         const int q = q0 + cl;
@@ -400,8 +401,8 @@ __device__ __forceinline__ float codes(const Args& A, const float4* gs, const fl
                         *reinterpret_cast<float4*>(A.y2 + ra[u] + Lg) = make_float4(a2[0].y, a2[1].y, a2[2].y, a2[3].y);
                         *reinterpret_cast<float4*>(A.y3 + ra[u] + Lg) = make_float4(0.f, a3[1].y, a3[2].y, a3[3].y);
                     }
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) absacc += fabsf(x[k].x) + fabsf(x[k].y);
+                    absacc += (double)((fabsf(x[0].x) + fabsf(x[1].x)) + (fabsf(x[2].x) + fabsf(x[3].x)));
+                    if (two) absacc += (double)((fabsf(x[0].y) + fabsf(x[1].y)) + (fabsf(x[2].y) + fabsf(x[3].y)));
                     continue;
                 }
                 float2 v[4], w[4];                                   // V; u (x becomes t)
@@ -585,9 +586,9 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_xc_codes(const __grid_consta
     }
     if (MODE != FIRST) load_w(A, ws, c);
     __syncthreads();
-    const float s = codes<MODE>(A, gs, ws, Vs, n, m0, Mr);
+    const double s = codes<MODE>(A, gs, ws, Vs, n, m0, Mr);
     __syncthreads();
-    if (MODE == LAST) block_sum((double)s, A.absx_part + n * A.G + g);
+    if (MODE == LAST) block_sum(s, A.absx_part + n * A.G + g);
     else convolve<false>(A, gs, Vs, A.P + (c * A.G + g) * A.Lg, Mr);
 }
 
@@ -630,7 +631,7 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_xc_all(const __grid_constant
     }
     load_w(A, ws, n);
     __syncthreads();
-    block_sum((double)codes<LAST>(A, gs, ws, Vs, n, 0, A.M), A.absx_part + n);
+    block_sum(codes<LAST>(A, gs, ws, Vs, n, 0, A.M), A.absx_part + n);
 }
 
 // The smallest n >= Lg of the form {1, 3, 5, 9, 15, 25} 2^a and its stages: the odd
