@@ -405,29 +405,47 @@ __device__ __forceinline__ bool last_block(unsigned* counter) {
 
 // Sums of many float32 terms.  A float64 sum per term is what bounds such a pass here (two
 // FP64 operations per SM and cycle: 13.2 ms for the threshold's two passes over 1.19e9
-// codes, 0.72 TB/s), so runs of 16 or 32 terms go into a compensated float32 pair first
-// (Knuth's two-sum: s + c is exact to about 2^-48 of the sum), and each run's pair into
-// float64.  Runs whose terms leave the range where that holds (products and their
-// errors neither overflow nor underflow) are summed in float64 term by term.
-__device__ __forceinline__ void add2(float& s, float& c, float x) {
-    const float t = __fadd_rn(s, x), b = __fsub_rn(t, s);
-    c = __fadd_rn(c, __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(x, b)));
-    s = t;
+// codes, 0.72 TB/s), so runs of 16 or 32 terms go into three float32 sums first, each of
+// the errors of the one before (Knuth's two-sum), and each run's sums into float64.  The
+// third one keeps what a pair loses, 2^-48 of a term: with a pair, the threshold was 4.6e-16
+// and the fit 9.7e-16 off 80-bit sums (rms; sizes of 2e5 to 8e6 codes), with three 7e-17 and
+// 8e-17, as with float64 per term.  Runs whose terms leave the range where that holds
+// (products and their errors neither overflow nor underflow) are summed in float64 term by
+// term.
+__device__ __forceinline__ float two_sum(float a, float b, float& err) {
+    const float t = __fadd_rn(a, b), x = __fsub_rn(t, a);
+    err = __fadd_rn(__fsub_rn(a, __fsub_rn(t, x)), __fsub_rn(b, x));
+    return t;
 }
-// (x - (mh + ml))^2, |ml| at most an ulp of mh, into the pair; returns |x - mh - ml|
-__device__ __forceinline__ float add_dev2(float& s, float& c, float x, float mh, float ml) {
-    const float d = __fsub_rn(x, mh), b = __fsub_rn(x, d);                 // x - mh = d + e
-    const float e = __fadd_rn(__fsub_rn(x, __fadd_rn(d, b)), __fsub_rn(b, mh));
-    const float lo = __fsub_rn(e, ml);
-    const float p = __fmul_rn(d, d);
-    float q = fmaf(d, d, -p);
-    q = fmaf(d + d, lo, q);
-    q = fmaf(lo, lo, q);
-    add2(s, c, p);
-    c += q;
-    return fabsf(d + lo);
-}
-constexpr float kDevMin = 1e-10f, kDevMax = 1e17f;     // deviations whose squares the pairs hold
+struct Sum3 {
+    float s = 0.f, c = 0.f, r = 0.f;
+    __device__ __forceinline__ void add_low(float x) {          // x at most the size of s's errors
+        float e;
+        c = two_sum(c, x, e);
+        r = __fadd_rn(r, e);
+    }
+    __device__ __forceinline__ void add(float x) {
+        float e;
+        s = two_sum(s, x, e);
+        add_low(e);
+    }
+    // (x - mh - ml)^2, |ml| at most an ulp of mh (MEAN; else zero); returns |x - mh - ml|
+    template <bool MEAN>
+    __device__ __forceinline__ float add_dev2(float x, float mh, float ml) {
+        float lo, lo2 = 0.f;
+        const float d = two_sum(x, -mh, lo);                    // x - mh = d + lo
+        if (MEAN) lo = two_sum(lo, -ml, lo2);
+        const float p = __fmul_rn(d, d), d2 = __fadd_rn(d, d), h = __fmul_rn(d2, lo);
+        add(p);
+        add_low(fmaf(d, d, -p));
+        add_low(h);
+        r = fmaf(lo, lo, __fadd_rn(r, fmaf(d2, lo, -h)));
+        if (MEAN) r = fmaf(d2, lo2, r);
+        return fabsf(d + lo);
+    }
+    __device__ __forceinline__ double total() const { return (double)s + ((double)c + (double)r); }
+};
+constexpr float kDevMin = 1e-10f, kDevMax = 1e17f;     // deviations whose squares the three sums hold
 
 // The objective: the sum over the data window of (DX - S)^2  (||W*DX - S||^2; rows of q4
 // float4s, window rows at gamma / 4 of the row of Lg / 4) into out by blocks; the last block
@@ -453,16 +471,17 @@ __global__ void k_fit(const float4* __restrict__ DX, const float4* __restrict__ 
                 b[u] = S[i];
             }
         }
-        float s = 0.f, c = 0.f, most = 0.f;
+        Sum3 run;
+        float most = 0.f;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            most = fmaxf(most, add_dev2(s, c, a[u].x, b[u].x, 0.f));
-            most = fmaxf(most, add_dev2(s, c, a[u].y, b[u].y, 0.f));
-            most = fmaxf(most, add_dev2(s, c, a[u].z, b[u].z, 0.f));
-            most = fmaxf(most, add_dev2(s, c, a[u].w, b[u].w, 0.f));
+            most = fmaxf(most, run.add_dev2<false>(a[u].x, b[u].x, 0.f));
+            most = fmaxf(most, run.add_dev2<false>(a[u].y, b[u].y, 0.f));
+            most = fmaxf(most, run.add_dev2<false>(a[u].z, b[u].z, 0.f));
+            most = fmaxf(most, run.add_dev2<false>(a[u].w, b[u].w, 0.f));
         }
-        if (most >= kDevMin && most <= kDevMax && s <= 1e36f) {
-            acc += (double)s + (double)c;
+        if (most >= kDevMin && most <= kDevMax && run.s <= 1e36f) {
+            acc += run.total();
         } else {
 #pragma unroll 1
             for (int u = 0; u < 4; ++u) {
@@ -487,7 +506,7 @@ __global__ void k_fit(const float4* __restrict__ DX, const float4* __restrict__ 
 
 // std of the positive entries: pass 1 (mu null) count + sum, pass 2 sum of squared
 // deviations from mu; 32 entries per run.  N = 20000, L = 200, K = 64 (4.75 GB a pass):
-// 13.2 ms for both passes with a float64 sum per entry, 2.65 ms with the runs.  The last block
+// 13.2 ms for both passes with a float64 sum per entry, 3.44 ms with the runs.  The last block
 // adds the partial sums: the count and mean to stat, or the deviation to the pinned host
 // scalar dev (two launches and a copy less: 48 -> 29 us with the wait at 200 x 10 x 232).
 constexpr int kPosBlocks = 152 * 4;
@@ -507,7 +526,8 @@ __global__ void __launch_bounds__(256) k_pos_stats(const float4* __restrict__ X,
 #pragma unroll
         for (int u = 0; u < U; ++u)
             v[u] = i0 + u * stride < n4 ? X[i0 + u * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
-        float s = 0.f, c = 0.f, most = 0.f;
+        Sum3 run;
+        float most = 0.f;
         unsigned pos = 0;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -517,19 +537,19 @@ __global__ void __launch_bounds__(256) k_pos_stats(const float4* __restrict__ X,
                 const bool on = e[k] > 0.f;
                 if (SECOND) {
                     // an entry that is not positive deviates by nothing
-                    most = fmaxf(most, add_dev2(s, c, on ? e[k] : mh, mh, on ? ml : 0.f));
+                    most = fmaxf(most, run.add_dev2<true>(on ? e[k] : mh, mh, on ? ml : 0.f));
                 } else {
-                    add2(s, c, on ? e[k] : 0.f);
+                    run.add(on ? e[k] : 0.f);
                 }
                 pos += on;
             }
         }
         count += pos;
-        const bool ok = SECOND ? mean_ok && s <= 1e36f &&
+        const bool ok = SECOND ? mean_ok && run.s <= 1e36f &&
                                      (pos == 0 || (most >= kDevMin && most >= 0.01f * fabsf(mh) && most <= kDevMax))
-                               : s <= 1e37f;
+                               : run.s <= 1e37f;
         if (ok) {
-            acc += (double)s + (double)c;
+            acc += run.total();
         } else {
 #pragma unroll 1
             for (int u = 0; u < U; ++u) {
