@@ -256,14 +256,16 @@ size_t dsolve_smem(int M, bool stage) {
 
 // launches k_dsolve for cn sequences, staging the spectra when they fit shared memory;
 // the new d-hat replaces Dh, times scale_out
+constexpr size_t kDsStage = 200 * 1024;
 int dsolve_launch(cdlgb_ctx* c, int cn, const float2* Yh, const float2* Hh, float2* Dh,
                   const float2* Zh, float2* Th, float scale_out) {
     const int F = c->F, M = c->M;
     const int nfb = (F + kDsBins - 1) / kDsBins;
     const size_t sm = dsolve_smem(M, true);
-    const bool stage = sm <= (size_t)200 * 1024;
+    const bool stage = sm <= kDsStage;
+    // process-wide per kernel: the same cap for every context
     if (stage && sm > 48 * 1024)
-        CU_TRY(c, cudaFuncSetAttribute(k_dsolve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        CU_TRY(c, cudaFuncSetAttribute(k_dsolve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDsStage));
     const dim3 g((unsigned)((size_t)nfb * cn)), b(kDsBins * kDsWarps);
     const float scale = 1.f / (float)c->Lg;
     if (stage)

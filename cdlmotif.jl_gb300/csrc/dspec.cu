@@ -500,18 +500,20 @@ int dspec_slots(int N, int chunk, int M, int F, int nsm) {
     return slots;
 }
 
-// NST buffers; the first D-step stages one spectrum of three, so twice as many sequences ahead
-template <int MW, int NST>
-static int launch(cdlgb_ctx* c, const SArgs& a, dim3 g) {
-    constexpr int deep = 2 * NST;
-    auto k = c->res_on ? (c->spec_init ? k_dspec<MW, deep, true, true> : k_dspec<MW, NST, true, false>)
-                       : (c->spec_init ? k_dspec<MW, deep, false, true> : k_dspec<MW, NST, false, false>);
-    const size_t sm = (size_t)2 * 5 * (kWarps + 1) * kBins * sizeof(float) +
-                      (size_t)(c->spec_init ? deep : 3 * NST) * MW * kBins * kWarps * sizeof(float2);
+template <int MW, int NST, bool INIT>
+static int launch_form(cdlgb_ctx* c, const SArgs& a, dim3 g) {
+    auto k = c->res_on ? k_dspec<MW, NST, true, INIT> : k_dspec<MW, NST, false, INIT>;
+    constexpr size_t sm = (size_t)2 * 5 * (kWarps + 1) * kBins * sizeof(float) +
+                          (size_t)(INIT ? 1 : 3) * NST * MW * kBins * kWarps * sizeof(float2);
     CU_TRY(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     k<<<g, kBins * kWarps, sm, c->stream>>>(a);
     LAUNCH_CHECK(c, "k_dspec");
     return CDLGB_OK;
+}
+// NST buffers; the first D-step stages one spectrum of three, so twice as many sequences ahead
+template <int MW, int NST>
+static int launch(cdlgb_ctx* c, const SArgs& a, dim3 g) {
+    return c->spec_init ? launch_form<MW, 2 * NST, true>(c, a, g) : launch_form<MW, NST, false>(c, a, g);
 }
 
 int dspec_launch(cdlgb_ctx* c, const float2* Yh, const float2* G3h, int c0, int c1, int slot0) {

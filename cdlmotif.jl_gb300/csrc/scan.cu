@@ -1146,7 +1146,7 @@ int touzet_thresholds(cdlgb_ctx* c, const float* pwms, const int32_t* lens, int 
     int32_t* d_alpha = c->scan_i + up;
     int32_t* d_status = d_alpha + K;
     CU_TRY(c, cudaMemcpyAsync(c->scan_i, host.data(), up * 4, cudaMemcpyHostToDevice, c->stream));
-    const int shm = (int)(2 * (size_t)kTouzetMaxR * sizeof(unsigned long long));
+    constexpr int shm = 2 * kTouzetMaxR * (int)sizeof(unsigned long long);
     CU_TRY(c, cudaFuncSetAttribute(k_touzet, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
     k_touzet<<<K, kTouzetThreads, shm, c->stream>>>(d_kq, d_kq + nk + 2 * (size_t)K, d_kq + nk, d_kq + nk + K, maxlen,
                                                     reinterpret_cast<const unsigned long long*>(c->scan_i), d_alpha,
