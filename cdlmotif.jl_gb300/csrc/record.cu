@@ -166,12 +166,13 @@ __global__ void __launch_bounds__(kTopoThreads) k_topology(
 // shifted by the pair's distance) and adds the code-weighted one-hot windows to its row
 // of shared memory, its lanes along the window; the warps' rows are added in order into
 // one partial per chunk (summed in order afterwards).
-constexpr int kMsaWarps = 8;                                  // at most: long spans take fewer
+constexpr int kMsaWarps = 8;
+constexpr int kMaxSpan = 1536;                                // k_pair_finish holds it in 48 KB of float64
 __global__ void __launch_bounds__(32 * kMsaWarps) k_pair_msa(
     const float* __restrict__ codes, const unsigned* __restrict__ mask, const float* __restrict__ S,
     const int* __restrict__ pairs, const int* __restrict__ kmap, const int* __restrict__ klen, int N, int M, int C,
     int max_span, float* __restrict__ part) {
-    extern __shared__ float acc[];                            // [warps][4 * max_span]
+    extern __shared__ float acc[];                            // [kMsaWarps][4 * max_span]
     const int p = blockIdx.x, ch = blockIdx.y, nch = gridDim.y;
     const int fr = pairs[3 * p] - 1, fc = pairs[3 * p + 1] - 1, o_len = pairs[3 * p + 2];
     const int fl1 = klen[fr], fl2 = klen[fc];
@@ -179,7 +180,7 @@ __global__ void __launch_bounds__(32 * kMsaWarps) k_pair_msa(
     const int t1 = kmap[fr] / M, f1 = kmap[fr] % M;
     const int t2 = kmap[fc] / M, f2 = kmap[fc] % M;
     const int words = (C + 31) / 32, ml = 4 * max_span;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* my = acc + warp * ml;
     for (int i = lane; i < ml; i += 32) my[i] = 0.f;
     __syncwarp();
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(32 * kMsaWarps) k_pair_msa(
     const int nl = 4 * span, sh = fl1 - o_len, sw = sh >> 5, sb = sh & 31;
     // fr starts at 0-based s, fc at s + sh; the window [s, s + span) inside the sequence
     const int last = C - span;
-    for (int n = n0 + warp; n < n1; n += nwarps) {
+    for (int n = n0 + warp; n < n1; n += kMsaWarps) {
         const size_t r1 = ((size_t)t1 * N + n) * M + f1, r2 = ((size_t)t2 * N + n) * M + f2;
         const unsigned* m1 = mask + r1 * words;
         const unsigned* m2 = mask + r2 * words;
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(32 * kMsaWarps) k_pair_msa(
     __syncthreads();
     for (int i = threadIdx.x; i < ml; i += blockDim.x) {
         float v = 0.f;
-        for (int w = 0; w < nwarps; ++w) v += acc[w * ml + i];
+        for (int w = 0; w < kMsaWarps; ++w) v += acc[w * ml + i];
         part[((size_t)p * nch + ch) * ml + i] = v;
     }
 }
@@ -423,6 +424,8 @@ int cdlgb_ar_pair_pfms(cdlgb_ar* a, cdlgb_ctx* c, const int32_t* pairs, int32_t 
     if (!c->loaded || c->N != a->N || c->L4 != 4 * a->C)
         return ar_err(a, CDLGB_EINVAL, "context does not hold the record's data");
     const int K = (int)a->uinds.size();
+    if (filter_size > (kMaxSpan + 1) / 2)
+        return ar_err(a, CDLGB_EINVAL, "filter size %d: pairs span at most %d bases", filter_size, kMaxSpan);
     const int max_span = 2 * filter_size - 1;   // extractions.jl:22
     for (int p = 0; p < P; ++p) {
         const int fr = pairs[3 * p], fc = pairs[3 * p + 1], o = pairs[3 * p + 2];
@@ -449,13 +452,11 @@ int cdlgb_ar_pair_pfms(cdlgb_ar* a, cdlgb_ctx* c, const int32_t* pairs, int32_t 
     int* dpairs = (int*)(dpfm + (size_t)P * 4 * max_span);
     int* dspan = dpairs + 3 * P;
     AR_CU(a, cudaMemcpyAsync(dpairs, pairs, 3 * (size_t)P * sizeof(int), cudaMemcpyHostToDevice, a->stream));
-    // as many warps as their rows of sums fit (process-wide cap, the same for every context)
-    constexpr int cap = 200 * 1024;
-    const size_t row = (size_t)4 * max_span * sizeof(float);
-    const int warps = std::max(1, (int)std::min<size_t>(kMsaWarps, cap / row));
-    const size_t sm = warps * row;
+    // (a process-wide cap, the same for every context)
+    constexpr int cap = kMsaWarps * 4 * kMaxSpan * (int)sizeof(float);
+    const size_t sm = (size_t)kMsaWarps * 4 * max_span * sizeof(float);
     if (sm > 48 * 1024) AR_CU(a, cudaFuncSetAttribute(k_pair_msa, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
-    k_pair_msa<<<dim3(P, nch), 32 * warps, sm, a->stream>>>(a->codes, a->mask, c->S, dpairs, a->kmap, a->klen,
+    k_pair_msa<<<dim3(P, nch), 32 * kMsaWarps, sm, a->stream>>>(a->codes, a->mask, c->S, dpairs, a->kmap, a->klen,
                                                                a->N, a->M, a->C, max_span, part);
     AR_CU(a, cudaGetLastError());
     k_pair_finish<<<P, 128, 4 * max_span * sizeof(double), a->stream>>>(part, dpairs, a->klen, P, nch,
