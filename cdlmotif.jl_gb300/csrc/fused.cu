@@ -769,7 +769,8 @@ int fused_autotune(cdlgb_ctx* c, int maxc, double* ms, int32_t* kind, int32_t* c
         if (st != CDLGB_OK) { free_all(-1); return st; }
         if (wp) cands.push_back({2, wp});
     }
-    if (c->xconv) cands.push_back({3, c->xconv});       // the convolution X-step, where it is in use
+    // the convolution X-step, where it is in use and the caller has room for it too
+    if (c->xconv && (int)cands.size() != maxc) cands.push_back({3, c->xconv});
     if (cands.empty()) return cdlgb_seterr(c, CDLGB_ENOTSUP, "autotune: no candidate");
     if ((int)cands.size() > maxc) {
         free_all(-1);
