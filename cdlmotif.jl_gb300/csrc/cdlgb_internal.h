@@ -242,6 +242,7 @@ int fused_autotune(cdlgb_ctx* c, int maxc, double* ms, int32_t* kind, int32_t* c
                    int32_t* n_out, int32_t* chosen);
 int fused_has_multi(cdlgb_ctx* c);
 int fused_multi_slots(cdlgb_ctx* c);      // filter slots of the multi-iteration kernel, 0 without one
+bool fused_one_step_regs(const cdlgb_ctx* c);   // whether the X-step is the one-X-step register-FFT kernel
 // ---- xconv.cu (X-steps by short convolutions) ----
 void* xconv_plan_create(cdlgb_ctx* c, int slots, int* status);
 void xconv_plan_free(cdlgb_ctx* c, void* p);

@@ -697,6 +697,11 @@ int fused_multi_slots(cdlgb_ctx* c) {
     return P && P->iter ? iter_plan_cluster(P->iter) * iter_plan_filters(P->iter) : 0;
 }
 
+bool fused_one_step_regs(const cdlgb_ctx* c) {
+    const FusedPlan* P = (const FusedPlan*)c->fplan;
+    return P && P->warp;
+}
+
 int fused_xsteps(cdlgb_ctx* c, const float* Xin, float* Xout, int iters) {
     FusedPlan* P = (FusedPlan*)c->fplan;
     return iter_xsteps(c, P->iter, Xin, Xout, iters);

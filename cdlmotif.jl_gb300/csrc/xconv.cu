@@ -816,27 +816,66 @@ void free_arrays(cdlgb_ctx* c, XconvPlan* P) {
 
 }  // namespace
 
-// Whether the automatic choice (fft_mode 0; 1 and 2 ask for the transforms) takes this X-step
-// for a context: every size without a multi-iteration register-FFT kernel (slots = 0), and
-// where that kernel's filter slots (16 per CTA, `slots` for all of M) are empty enough.
-// Measured per X-step and code value, N = 500-20000: 4.4-5.2 ps per slot for the register
-// FFTs, 5.8 / 7.7 / 7.1 ps per filter (an odd M counts one more) for these kernels at
-// T = 16 / 48 / 64 taps; 9.3-11.5 ps for the in-kernel mixed-radix FFTs and 16 ps for the
-// cuFFT transforms.  CDLGB_XCONV=0 and the switches that pick an FFT form leave it out.
-static int xconv_wanted(const cdlgb_ctx* c, int slots) {
+// Whether the automatic choice (fft_mode 0; 1 and 2 ask for the transforms) may take this
+// X-step for a context.  CDLGB_XCONV=0 and the switches that pick an FFT form leave it out.
+static bool xconv_allowed(const cdlgb_ctx* c) {
     const int T = 4 * c->p.filter_size, TP = (T + 15) / 16 * 16;
-    if (c->p.fft_mode != 0 || T > kMaxTaps || c->Lg % 4 || c->Lg > kMaxLg || c->Lg < TP) return 0;
-    if (getenv("CDLGB_GENERIC_FFT")) return 0;
+    if (c->p.fft_mode != 0 || T > kMaxTaps || c->Lg % 4 || c->Lg > kMaxLg || c->Lg < TP) return false;
+    if (getenv("CDLGB_GENERIC_FFT")) return false;
     for (const char* v : {"CDLGB_XCONV", "CDLGB_XITER"}) {
         const char* e = getenv(v);
-        if (e && atoi(e) == 0) return 0;
+        if (e && atoi(e) == 0) return false;
     }
-    return slots == 0 || (c->M + 1) / 2 * 2 * (5.5 + 0.03 * T) < 4.8 * slots;
+    return true;
+}
+
+// Whether it is the cheaper one, by estimates in ps per X-step and code value from 2300
+// measured sizes (Lg = 40-12288, M = 1-256, T = 4-128, 2 to 6e7 code values; 15 X-steps each
+// way).  The number of sequences has no say: a sequence's route, and with it its bits, must
+// not depend on how many others there are.
+//   * these kernels, 8 % rms: the taps, filled up to 16s, in lanes of which 1 / pad have work
+//     (short rows are not bound by that); the element-wise pass; the solve, a transform per
+//     sequence; 2.5 where two CTAs per SM leave each one pair of filters, 6 where one CTA
+//     fits.  M = 32, T = 64: 6.6 measured at Lg = 512, 7.3 at 2048, 8.7 at 4224, 10.1 at 5120,
+//     12.6 at 8192; M = 9: 9.5, 9.9, 11.2, 10.9, 14.3;
+//   * the multi-iteration register-FFT kernel (slots: its filter slots for all of M, 16 per
+//     CTA), per slot: 4.5-5.0, 4.8-5.6 with three CTAs or more, 4.2-4.8 up to 8 filters in
+//     one, 3.6-4.0 with 32 lanes per transform.  M = 10: 7.4 at Lg = 928, where these kernels
+//     take 5.5 with T = 16 and 9.0 with T = 64.  A tenth less is granted, which these kernels
+//     lose with a few hundred sequences (Lg = 832, M = 18, T = 48: 0.97 of that kernel's speed
+//     with 1300 sequences, 0.87 with 670); left alone where M (5.5 + 0.03 T) is above 4.8 per
+//     slot, the two being close there;
+//   * the other transforms, from below: the one-X-step register FFTs (M = 33: 7.5, 17: 7.9, 9:
+//     8.4, 5: 9.7); the in-kernel mixed radix (10.0 at Lg = 1024, 11-19 elsewhere, 15 and more
+//     at M = 5); cuFFT by the largest prime factor of Lg (M = 32: 9.5 at 2048 and 4096; 12.2-19
+//     up to 19; 14.7-24 up to 47; 21-65 past it).
+static bool xconv_cheaper(const cdlgb_ctx* c, const Shape& s, int n, int slots) {
+    const int T = 4 * c->p.filter_size, Lg = c->Lg;
+    const double M = c->M;
+    double pad = 64.0 * s.G * ((s.nchunk + s.CG - 1) / s.CG) / (s.nchunk * M);
+    if (Lg < 320) pad = std::min(pad, 1.5);
+    const bool two = 2 * (s.smem + 1024) <= kSmemSm;
+    const double room = !two ? 6.0 : s.B == 1 && c->M > 2 ? 2.5 : 0.0;
+    const double conv = 1.3 + pad * (1.63 + 0.0594 * 16 * s.NB) + 16.0 * n / (Lg * M) + room;
+    if (slots) {
+        const double per_slot = c->M > 8 ? (slots <= 32 ? 4.0 : 4.4) : Lg < 520 ? 4.0 : 3.4;
+        return M * (5.5 + 0.03 * T) < 4.8 * slots && conv < per_slot * slots / M;
+    }
+    int odd = Lg, most = 1;
+    while (odd % 2 == 0) odd /= 2;
+    for (int p = 3; odd > 1; p += 2)
+        for (; odd % p == 0; odd /= p) most = p;
+    double fft;
+    if (fused_one_step_regs(c)) fft = 7.2 + 10 / M + 9 / (M * M);
+    else if (c->fused) fft = (Lg == 1024 ? 10.0 : 11.5) + (c->M < 9 ? 15 / M + 15 / (M * M) : 0.0);
+    else if (most == 1) fft = 8.5 + 8.5 / M;
+    else fft = (most <= 19 ? 11.0 : most <= 47 ? 14.0 : 20.0) + 11 / M;
+    return conv < fft;
 }
 
 void* xconv_plan_create(cdlgb_ctx* c, int slots, int* status) {
     *status = CDLGB_OK;
-    if (!xconv_wanted(c, slots)) return nullptr;
+    if (!xconv_allowed(c)) return nullptr;
     const int Lg = c->Lg;
     XconvPlan* P = new XconvPlan();
     P->n = transform_length(Lg, P->radix, &P->nst);
@@ -844,7 +883,7 @@ void* xconv_plan_create(cdlgb_ctx* c, int slots, int* status) {
     P->solve_smem = (size_t)(n + n / 16 + 1) * sizeof(float2);
     P->solve_threads = n <= 512 ? 64 : n <= 1536 ? 128 : 256;
     const int T = 4 * c->p.filter_size;
-    if (P->solve_smem > kSmemCta || !choose_shape(Lg, c->M, T, n, &P->s)) {
+    if (P->solve_smem > kSmemCta || !choose_shape(Lg, c->M, T, n, &P->s) || !xconv_cheaper(c, P->s, n, slots)) {
         delete P;
         return nullptr;
     }
@@ -853,9 +892,13 @@ void* xconv_plan_create(cdlgb_ctx* c, int slots, int* status) {
     P->PCG = P->s.CG;
     // the parts of P lie in the cuFFT passes' scratch
     P->chunk = (int)std::min<size_t>((size_t)c->chunk * c->M / P->G, c->N);
-    // one CTA per sequence where that keeps every sequence resident (M <= 32)
+    // One CTA per sequence (M <= 32) where that keeps every sequence resident and a
+    // sequence's work, one CTA's chain, is short.  15 X-steps of 30 sequences, so and with a
+    // launch per part: 0.17 and 0.27 ms at Lg = 436, M = 16, T = 16 (0.4 million in the rule's
+    // units), 0.47 / 0.44 at 1060, 16, 64 (1.9), 0.59 / 0.45 at 1456, 32, 16 (3.0), 1.18 / 0.72
+    // at 4096, 9, 64 (4.1); of 200 sequences: 0.51 / 0.61 at 1456, 16, 16 (1.5).
     P->all = false;
-    if (c->M <= 32 && P->chunk == c->N) {
+    if (c->M <= 32 && P->chunk == c->N && (long long)c->M * Lg * (48 + T) <= 2000000) {
         Shape a = shape_for(Lg, c->M, T, 16, n);
         // as few warps as finish both passes (codes, parts of P) in the fewest rounds
         const int codes_n = (a.nchunk + a.CG - 1) / a.CG, parts_n = P->G * ((a.nchunk + P->PCG - 1) / P->PCG);
