@@ -516,6 +516,14 @@ def _any_entry(pos: np.ndarray) -> np.ndarray:
     return pos.max(axis=0, initial=0) > 0
 
 
+def _hit_counts(positions) -> np.ndarray:
+    """Per motif the number of entries (> 0) of positions (N, K).  Integers are summed without
+    a boolean array; anything else (a fraction, a NaN) is compared."""
+    pos = np.asarray(positions)
+    on = np.clip(pos, 0, 1) if pos.dtype.kind in "iu" else pos > 0
+    return on.sum(axis=0, dtype=np.int32)
+
+
 def _columns(a: np.ndarray, keep: np.ndarray) -> np.ndarray:
     """The kept motifs' columns of an array of this module's own, as a C-order array (take
     is faster than a boolean column index, and needs no bounds checks here)."""
@@ -660,8 +668,8 @@ def filter_using_evalue(c: CDL, pwms, thresh, positions, lens=None, cpu=False, n
             bg_pos, bg_sc, _ = overlapping_scan(c, pwms, thresh, ln)
             if non_overlap:
                 bg_pos, _, _ = non_overlap_scan(c, bg_pos, bg_sc, ln, None)
-    hits = np.clip(positions, 0, 1).sum(axis=0, dtype=np.int32)
-    hits_bg = np.clip(bg_pos, 0, 1).sum(axis=0, dtype=np.int32)
+    hits = _hit_counts(positions)
+    hits_bg = _hit_counts(bg_pos)
     ev = fisher_evalues(hits, hits_bg, c.N)
     if get_evalues_only:
         return ev
