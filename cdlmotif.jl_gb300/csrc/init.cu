@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kNT, 3) k_init_x(XArgs A) {
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
     const size_t items = (size_t)A.N * A.nr;
     float s = 0.f, sc = 0.f;
-    double total = 0.0;
+    double total = 0.0, rest = 0.0;
     for (size_t item = blockIdx.x; item < items; item += gridDim.x) {
         const size_t n = item / A.nr;
         const int a0 = (int)(item - n * A.nr) * A.RA, an = min(A.RA, A.La - a0);
@@ -150,10 +150,18 @@ __global__ void __launch_bounds__(kNT, 3) k_init_x(XArgs A) {
                             }
                             if (i >= Hp && t0 == 0) {      // the range's own
                                 A.X[j] = make_float4(v, 0.f, 0.f, 0.f);
-                                // sum |X| as a compensated pair (two-sum)
-                                const float x = fabsf(v), t = __fadd_rn(s, x), b = __fsub_rn(t, s);
-                                sc = __fadd_rn(sc, __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(x, b)));
-                                s = t;
+                                // sum |X| (two-sum): drawn codes as a float32 pair per
+                                // range, which for them has the bits of a float64 sum;
+                                // given ones, of any size, as a float64 pair
+                                if (DRAW) {
+                                    const float x = fabsf(v), t = __fadd_rn(s, x), b = __fsub_rn(t, s);
+                                    sc = __fadd_rn(sc, __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(x, b)));
+                                    s = t;
+                                } else {
+                                    const double x = (double)fabsf(v), t = total + x, b = t - total;
+                                    rest += (total - (t - b)) + (x - b);
+                                    total = t;
+                                }
                             }
                         }
                         xs[mm * A.pitch + place(i)] = v;
@@ -223,9 +231,10 @@ __global__ void __launch_bounds__(kNT, 3) k_init_x(XArgs A) {
             A.DX[j] = v;
             A.G2[j] = v;
         }
-        total += (double)s + (double)sc;
+        if (DRAW) total += (double)s + (double)sc;
         s = sc = 0.f;
     }
+    total += rest;
     for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
     __syncthreads();
     if (lane == 0) sh[warp] = total;
