@@ -543,7 +543,11 @@ def extend(c: CDL, positions, lens, filter_size: int, use_comp=None, bg=_BG, pse
     keep = _any_entry(pos) & (ln > filter_size + 2)
     pos = _columns(pos, keep)
     ln = ln[keep]
-    uc = None if use_comp is None else np.asarray(use_comp).take(np.flatnonzero(keep), axis=1)
+    uc = None if use_comp is None else np.asarray(use_comp)
+    if uc is not None and uc.shape[1:] == keep.shape:    # a column per motif: no index out of range
+        uc = np.array(uc, order="C") if keep.all() else _columns(uc, keep)
+    elif uc is not None:
+        uc = uc.take(np.flatnonzero(keep), axis=1)
     pfms = None
     if re_evaluate_pfm:
         pfms = posdicts2pfms(c, pos, ln, uc, pseudocounts_r, pseudocount, smoothing) if len(ln) else []
