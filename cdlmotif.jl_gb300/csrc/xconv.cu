@@ -829,29 +829,34 @@ static bool xconv_allowed(const cdlgb_ctx* c) {
     return true;
 }
 
-// Whether it is the cheaper one, by estimates in ps per X-step and code value from 2300
-// measured sizes (Lg = 40-12288, M = 1-256, T = 4-128, 2 to 6e7 code values; 15 X-steps each
-// way).  The number of sequences has no say: a sequence's route, and with it its bits, must
-// not depend on how many others there are.
+// Whether an allowed context takes it.  Up to 64 taps and Lg = 4128: every length without a
+// multi-iteration register-FFT kernel (slots: its filter slots for all of M, 16 per CTA; else
+// 0), and where those slots are empty enough, 5.5 + 0.03 T ps per filter against 4.8 per slot.
+// It is the more exact form there (32 trainings of 16 sizes, after one outer iteration against
+// float64: DX 2 to 20 times nearer than by the transforms, codes 2 to 6) and mostly the faster
+// one; where it is not (0.79 to 0.95 of the transforms' speed: M = 8, 10 with W = 16 at L = 200;
+// odd M at Lg = 496 and 928; M = 9 at Lg = 4096) the more exact one is kept.  Past those sizes
+// the cheaper one is taken, by estimates in ps per X-step and code value from 2300 measured
+// sizes (Lg = 40-12288, M = 1-256, T = 4-128, 2 to 6e7 code values; 15 X-steps each way).  The
+// number of sequences has no say: a sequence's route, and with it its bits, must not depend
+// on how many others there are.
 //   * these kernels, 8 % rms: the taps, filled up to 16s, in lanes of which 1 / pad have work
 //     (short rows are not bound by that); the element-wise pass; the solve, a transform per
 //     sequence; 2.5 where two CTAs per SM leave each one pair of filters, 6 where one CTA
 //     fits.  M = 32, T = 64: 6.6 measured at Lg = 512, 7.3 at 2048, 8.7 at 4224, 10.1 at 5120,
 //     12.6 at 8192; M = 9: 9.5, 9.9, 11.2, 10.9, 14.3;
-//   * the multi-iteration register-FFT kernel (slots: its filter slots for all of M, 16 per
-//     CTA), per slot: 4.5-5.0, 4.8-5.6 with three CTAs or more, 4.2-4.8 up to 8 filters in
-//     one, 3.6-4.0 with 32 lanes per transform.  M = 10: 7.4 at Lg = 928, where these kernels
-//     take 5.5 with T = 16 and 9.0 with T = 64.  A tenth less is granted, which these kernels
-//     lose with a few hundred sequences (Lg = 832, M = 18, T = 48: 0.97 of that kernel's speed
-//     with 1300 sequences, 0.87 with 670); left alone where M (5.5 + 0.03 T) is above 4.8 per
-//     slot, the two being close there;
+//   * the multi-iteration register-FFT kernel, per slot: 4.5-5.0, 4.8-5.6 with three CTAs or
+//     more, 4.2-4.8 up to 8 filters in one, 3.6-4.0 with 32 lanes per transform.  A tenth less
+//     is granted, which these kernels lose with a few hundred sequences;
 //   * the other transforms, from below: the one-X-step register FFTs (M = 33: 7.5, 17: 7.9, 9:
 //     8.4, 5: 9.7); the in-kernel mixed radix (10.0 at Lg = 1024, 11-19 elsewhere, 15 and more
 //     at M = 5); cuFFT by the largest prime factor of Lg (M = 32: 9.5 at 2048 and 4096; 12.2-19
 //     up to 19; 14.7-24 up to 47; 21-65 past it).
-static bool xconv_cheaper(const cdlgb_ctx* c, const Shape& s, int n, int slots) {
+static bool xconv_wanted(const cdlgb_ctx* c, const Shape& s, int n, int slots) {
     const int T = 4 * c->p.filter_size, Lg = c->Lg;
     const double M = c->M;
+    const bool empty = (c->M + 1) / 2 * 2 * (5.5 + 0.03 * T) < 4.8 * slots;
+    if (T <= 64 && Lg <= 4128) return slots == 0 || empty;
     double pad = 64.0 * s.G * ((s.nchunk + s.CG - 1) / s.CG) / (s.nchunk * M);
     if (Lg < 320) pad = std::min(pad, 1.5);
     const bool two = 2 * (s.smem + 1024) <= kSmemSm;
@@ -859,7 +864,7 @@ static bool xconv_cheaper(const cdlgb_ctx* c, const Shape& s, int n, int slots) 
     const double conv = 1.3 + pad * (1.63 + 0.0594 * 16 * s.NB) + 16.0 * n / (Lg * M) + room;
     if (slots) {
         const double per_slot = c->M > 8 ? (slots <= 32 ? 4.0 : 4.4) : Lg < 520 ? 4.0 : 3.4;
-        return M * (5.5 + 0.03 * T) < 4.8 * slots && conv < per_slot * slots / M;
+        return empty && conv < per_slot * slots / M;
     }
     int odd = Lg, most = 1;
     while (odd % 2 == 0) odd /= 2;
@@ -883,7 +888,7 @@ void* xconv_plan_create(cdlgb_ctx* c, int slots, int* status) {
     P->solve_smem = (size_t)(n + n / 16 + 1) * sizeof(float2);
     P->solve_threads = n <= 512 ? 64 : n <= 1536 ? 128 : 256;
     const int T = 4 * c->p.filter_size;
-    if (P->solve_smem > kSmemCta || !choose_shape(Lg, c->M, T, n, &P->s) || !xconv_cheaper(c, P->s, n, slots)) {
+    if (P->solve_smem > kSmemCta || !choose_shape(Lg, c->M, T, n, &P->s) || !xconv_wanted(c, P->s, n, slots)) {
         delete P;
         return nullptr;
     }
