@@ -512,14 +512,22 @@ __global__ void __launch_bounds__(32 * kLutWarps, 2) k_scan_lut(const __grid_con
         const float* col = A.data + (size_t)n * 4 * L;
         bool odd = false;
         __syncwarp();
-        for (int v = 0; v <= words; ++v) {
-            const int l = 32 * v + lane;
-            const unsigned b = l < L ? base_bits(col, l) : 0u;
-            odd |= l < L && (b == 0 || (b & (b - 1)) != 0);
+        for (int v0 = 0; v0 <= words; v0 += 4) {
+            unsigned b[4];                                            // four words' loads in flight
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const unsigned m = __ballot_sync(full, b >> j & 1);
-                if (lane == j) planes[j * (words + 1) + v] = m;
+            for (int u = 0; u < 4; ++u) {
+                const int l = 32 * (v0 + u) + lane;
+                b[u] = l < L ? base_bits(col, l) : 0u;
+                odd |= l < L && (b[u] == 0 || (b[u] & (b[u] - 1)) != 0);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (v0 + u > words) break;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const unsigned m = __ballot_sync(full, b[u] >> j & 1);
+                    if (lane == j) planes[j * (words + 1) + v0 + u] = m;
+                }
             }
         }
         odd = __any_sync(full, odd);
@@ -706,13 +714,13 @@ int check_pwm_args(cdlgb_ctx* c, const float* pwms, const int32_t* lens, const f
 
 // The filtered scans take motifs of at most 32 columns and sequences of at most 4096 bases;
 // the forward scan's threshold is not negative (below zero its first maximum can be a
-// window that is no hit).  Fills the motifs' scales and limits (as floats' bits), the
+// window that is no hit).  Fills the motifs' thresholds, scales and limits (as floats' bits), the
 // motifs per CTA and the widest motif's columns: the array may be wider than any of them
 // (zero padding up to maxlen), and the tables go by the motifs alone.
 bool lut_ok(const cdlgb_ctx* c, const float* pwms, const int32_t* lens, const float* thresh, int K, int maxlen,
             bool both, std::vector<float>& meta, int* KG, int* widest) {
     if (maxlen > 32 || c->L4 / 4 > 4096 || !sparse_ok(c, pwms, lens, K, maxlen)) return false;
-    meta.resize(2 * (size_t)K);
+    meta.resize(3 * (size_t)K);
     int segs = 0, most = 1;
     *widest = 1;
     for (int k = 0; k < K; ++k) {
@@ -727,12 +735,13 @@ bool lut_ok(const cdlgb_ctx* c, const float* pwms, const int32_t* lens, const fl
         if (!(S < 1e30) || (S > 0.0 && S < 1e-25)) return false;
         const int ns = (lens[k] + 3) / 4;
         const float scale = S > 0.0 ? (float)(32000.0 / S) : 0.f;
-        meta[k] = scale;
+        meta[k] = thresh[k];
+        meta[K + k] = scale;
         const double at = floor((double)scale * (double)thresh[k]) + 32768.0 - (ns / 2 + 1);
         // a NaN threshold has no hit; a motif of zeros is left to the exact sums
         const int32_t limit = thresh[k] != thresh[k] ? 65536 : scale == 0.f ? 1
                             : at > 65536.0 ? 65536 : at < 1.0 ? 1 : (int32_t)at;
-        memcpy(&meta[K + k], &limit, 4);
+        memcpy(&meta[2 * (size_t)K + k], &limit, 4);
         segs += ns;
         most = std::max(most, ns);
         *widest = std::max(*widest, (int)lens[k]);
@@ -742,36 +751,42 @@ bool lut_ok(const cdlgb_ctx* c, const float* pwms, const int32_t* lens, const fl
     return true;
 }
 
-// device scratch layout: [pwms K*4*maxlen f32][thresh K f32] and [lens K i32][pos K*N i32]
-int upload_pwms(cdlgb_ctx* c, const float* pwms, const int32_t* lens, const float* thresh, int K,
-                int maxlen, size_t extra_i) {
-    size_t nf = (size_t)K * 4 * maxlen + K;
-    ST_TRY(ensure_scratch(c, &c->scan_f, &c->scan_f_cap, nf + (size_t)K * c->N + 2 * (size_t)K));
+// device scratch layout: [pwms K*4*maxlen f32][per motif, 3 K f32: the threshold, and for the
+// filtered scans what lut_ok fills][scores K*N f32] and [lens K i32][pos K*N i32]
+int upload_pwms(cdlgb_ctx* c, const float* pwms, const int32_t* lens, const float* thresh,
+                const std::vector<float>& meta, int K, int maxlen, size_t extra_i) {
+    const size_t np = (size_t)K * 4 * maxlen;
+    ST_TRY(ensure_scratch(c, &c->scan_f, &c->scan_f_cap, np + 3 * (size_t)K + (size_t)K * c->N));
     ST_TRY(ensure_scratch(c, &c->scan_i, &c->scan_i_cap, (size_t)K + extra_i));
-    CU_TRY(c, cudaMemcpyAsync(c->scan_f, pwms, (size_t)K * 4 * maxlen * 4, cudaMemcpyHostToDevice,
-                              c->stream));
-    CU_TRY(c, cudaMemcpyAsync(c->scan_f + (size_t)K * 4 * maxlen, thresh, (size_t)K * 4,
-                              cudaMemcpyHostToDevice, c->stream));
+    CU_TRY(c, cudaMemcpyAsync(c->scan_f, pwms, np * 4, cudaMemcpyHostToDevice, c->stream));
+    if (meta.empty())
+        CU_TRY(c, cudaMemcpyAsync(c->scan_f + np, thresh, (size_t)K * 4, cudaMemcpyHostToDevice, c->stream));
+    else
+        CU_TRY(c, cudaMemcpyAsync(c->scan_f + np, meta.data(), meta.size() * 4, cudaMemcpyHostToDevice, c->stream));
     CU_TRY(c, cudaMemcpyAsync(c->scan_i, lens, (size_t)K * 4, cudaMemcpyHostToDevice, c->stream));
     return CDLGB_OK;
 }
 
-// The filtered scan of one or both strands; dmeta: 2 K floats of device scratch.  Shared
-// memory: KG ceil(widest / 4) <= kLutSegs KB of tables, at most 33 KB of planes (4096
-// bases) and KG 16 widest <= 6.5 KB of motifs.
+// The filtered scan of one or both strands.  Shared memory: KG ceil(widest / 4) <= kLutSegs KB
+// of tables, at most 33 KB of planes (4096 bases) and KG 16 widest <= 6.5 KB of motifs.  A warp
+// takes a sequence, so few sequences leave SMs idle and a warp's motifs in a row are the
+// time: there the motifs are cut further, as long as the CTAs are no more than two per SM
+// (500 sequences of 4000, 24 motifs: 1.21 -> 0.37 ms for the forward call; 20 of 1000, 8 motifs:
+// 0.139 -> 0.073).
 template <bool BOTH>
-int launch_lut(cdlgb_ctx* c, const std::vector<float>& meta, int KG, int widest, int K, int maxlen, int32_t* dpos,
-               float* dscore, uint8_t* dcomp, float* dmeta) {
-    CU_TRY(c, cudaMemcpyAsync(dmeta, meta.data(), (size_t)K * 8, cudaMemcpyHostToDevice, c->stream));
+int launch_lut(cdlgb_ctx* c, int KG, int widest, int K, int maxlen, int32_t* dpos, float* dscore, uint8_t* dcomp) {
     LutArgs a;
     a.data = scan_data(c); a.pwms = c->scan_f; a.lens = c->scan_i; a.thresh = c->scan_f + (size_t)K * 4 * maxlen;
-    a.scale = dmeta; a.limit = reinterpret_cast<const int32_t*>(dmeta + K); a.pos = dpos; a.score = dscore; a.comp = dcomp;
+    a.scale = a.thresh + K; a.limit = reinterpret_cast<const int32_t*>(a.thresh + 2 * (size_t)K);
+    a.pos = dpos; a.score = dscore; a.comp = dcomp;
+    const int blocks = (c->N + kLutWarps - 1) / kLutWarps, cut = std::min(K, 2 * 152 / blocks);
+    if (cut > 1) KG = std::min(KG, (K + cut - 1) / cut);
     a.K = K; a.KG = KG; a.widest = widest; a.L = c->L4 / 4; a.N = c->N; a.words = (a.L + 31) / 32;
     const size_t shm = (size_t)KG * ((widest + 3) / 4) * 1024 + (size_t)kLutWarps * 16 * (a.words + 1) +
                        (size_t)KG * 16 * widest;
     CU_TRY(c, cudaFuncSetAttribute(k_scan_lut<BOTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 150 * 1024));
     const int parts = (K + KG - 1) / KG;
-    const int gx = std::max(1, std::min((c->N + kLutWarps - 1) / kLutWarps, 2 * 152 / parts));
+    const int gx = std::max(1, std::min(blocks, 2 * 152 / parts));
     k_scan_lut<BOTH><<<dim3(gx, parts), 32 * kLutWarps, shm, c->stream>>>(a);
     LAUNCH_CHECK(c, "k_scan_lut");
     return CDLGB_OK;
@@ -784,7 +799,11 @@ int scan_fwd(cdlgb_ctx* c, const float* pwms, const int32_t* lens, const float* 
     ST_TRY(check_pwm_args(c, pwms, lens, thresh, K, maxlen));
     const int N = c->N, L = c->L4 / 4;
     cdlgb_phase_begin(c, PH_SCAN);
-    ST_TRY(upload_pwms(c, pwms, lens, thresh, K, maxlen, (size_t)K * N));
+    std::vector<float> meta;
+    int KG = 0, widest = 0;
+    const bool lut = lut_ok(c, pwms, lens, thresh, K, maxlen, false, meta, &KG, &widest);
+    if (!lut) meta.clear();
+    ST_TRY(upload_pwms(c, pwms, lens, thresh, meta, K, maxlen, (size_t)K * N));
     int32_t* dpos = c->scan_i + K;
     size_t shm = (size_t)4 * L * sizeof(float);
     if (shm > 200 * 1024) return cdlgb_seterr(c, CDLGB_ENOTSUP, "scan: L=%d too long", L);
@@ -793,11 +812,8 @@ int scan_fwd(cdlgb_ctx* c, const float* pwms, const int32_t* lens, const float* 
     const int nts = ((L + 31) / 32) * 32;
     const size_t shs = (size_t)K * 4 * maxlen * sizeof(float) + (size_t)K * (nts / 32) * sizeof(VI) +
                        (size_t)L;
-    std::vector<float> meta;
-    int KG = 0, widest = 0;
-    if (lut_ok(c, pwms, lens, thresh, K, maxlen, false, meta, &KG, &widest)) {
-        ST_TRY(launch_lut<false>(c, meta, KG, widest, K, maxlen, dpos, nullptr, nullptr,
-                                 c->scan_f + (size_t)K * 4 * maxlen + K + (size_t)K * N));
+    if (lut) {
+        ST_TRY(launch_lut<false>(c, KG, widest, K, maxlen, dpos, nullptr, nullptr));
     } else if (nts <= 1024 && shs <= 64 * 1024 && sparse_ok(c, pwms, lens, K, maxlen)) {
         if (shs > 48 * 1024)
             CU_TRY(c, cudaFuncSetAttribute(k_scan_fwd_sparse, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -825,10 +841,14 @@ int scan_both(cdlgb_ctx* c, const float* pwms, const int32_t* lens, const float*
     ST_TRY(check_pwm_args(c, pwms, lens, thresh, K, maxlen));
     const int N = c->N, L = c->L4 / 4;
     cdlgb_phase_begin(c, PH_SCAN);
-    ST_TRY(upload_pwms(c, pwms, lens, thresh, K, maxlen, (size_t)K * N));
+    std::vector<float> meta;
+    int KG = 0, widest = 0;
+    const bool lut = lut_ok(c, pwms, lens, thresh, K, maxlen, true, meta, &KG, &widest);
+    if (!lut) meta.clear();
+    ST_TRY(upload_pwms(c, pwms, lens, thresh, meta, K, maxlen, (size_t)K * N));
     ST_TRY(ensure_scratch(c, &c->scan_u, &c->scan_u_cap, (size_t)K * N));
     int32_t* dpos = c->scan_i + K;
-    float* dscore = c->scan_f + (size_t)K * 4 * maxlen + K;
+    float* dscore = c->scan_f + (size_t)K * 4 * maxlen + 3 * (size_t)K;
     size_t shm = (size_t)4 * L * sizeof(float);
     if (shm > 200 * 1024) return cdlgb_seterr(c, CDLGB_ENOTSUP, "scan: L=%d too long", L);
     // one position per thread and the staged PWMs when they fit: at most 1024 positions
@@ -838,10 +858,8 @@ int scan_both(cdlgb_ctx* c, const float* pwms, const int32_t* lens, const float*
                        (size_t)4 * L * sizeof(float);
     const size_t shp = (size_t)K * 4 * maxlen * sizeof(float2) + (size_t)K * (nts / 32) * 2 * sizeof(VI) +
                        (size_t)4 * ((L + 31) / 32 + 2) * sizeof(uint32_t);
-    std::vector<float> meta;
-    int KG = 0, widest = 0;
-    if (lut_ok(c, pwms, lens, thresh, K, maxlen, true, meta, &KG, &widest)) {
-        ST_TRY(launch_lut<true>(c, meta, KG, widest, K, maxlen, dpos, dscore, c->scan_u, dscore + (size_t)K * N));
+    if (lut) {
+        ST_TRY(launch_lut<true>(c, KG, widest, K, maxlen, dpos, dscore, c->scan_u));
     } else if (nts <= 1024 && maxlen <= 64 && shp <= 64 * 1024 && sparse_ok(c, pwms, lens, K, maxlen)) {
         if (shp > 48 * 1024)
             CU_TRY(c, cudaFuncSetAttribute(k_scan_both_sparse, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
