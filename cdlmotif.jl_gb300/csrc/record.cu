@@ -30,7 +30,7 @@ struct cdlgb_ar {
     int* anym = nullptr;                                     // (M) scratch
     int* kmap = nullptr;                                     // (Kcap) t*M + m
     int* klen = nullptr;                                     // (Kcap) filter length (bases)
-    unsigned* mask = nullptr;                                // (T, N, M, ceil(C/32)): codes > thresh[t]
+    unsigned* mask = nullptr;                                // (T, N, M, ceil(C/32)): codes > thresh[t]; behind codes
     int* dcount = nullptr;                                   // topology outputs (device)
     size_t dcount_cap = 0;
     float* msa = nullptr;                                    // pair MSA partials
@@ -57,23 +57,37 @@ int ar_err(cdlgb_ar* a, int code, const char* fmt, ...) {
     } while (0)
 
 // codes[t] <- X_best rows gamma, gamma+4, ...; the bits code > thresh; anym[m] |= any.
-// One warp per row (n, m).  X_best is read whole (its sectors hold 8 rows each).
+// A warp takes 256 positions of a row (n, m), their loads in flight together; long rows of
+// few sequences so spread over the warps too (two records of 50 x 8 rows of 20000, with the
+// allocations: 844 us with a warp per row and a word at a time, 399 so).
+// X_best is read whole (its sectors hold 8 rows each).
+constexpr int kRecWords = 8;
 __global__ void __launch_bounds__(256) k_record(const float* __restrict__ Xb, float* __restrict__ codes,
                                                 unsigned* __restrict__ mask, size_t rows, int M, int C, int Lg,
                                                 int gamma, float thresh, int* __restrict__ anym) {
-    const int lane = threadIdx.x & 31, words = (C + 31) / 32;
+    const int lane = threadIdx.x & 31, words = (C + 31) / 32, segs = (words + kRecWords - 1) / kRecWords;
     const size_t stride = (size_t)gridDim.x * (blockDim.x / 32);
-    for (size_t r = blockIdx.x * (size_t)(blockDim.x / 32) + (threadIdx.x >> 5); r < rows; r += stride) {
+    for (size_t i = blockIdx.x * (size_t)(blockDim.x / 32) + (threadIdx.x >> 5); i < rows * segs; i += stride) {
+        const size_t r = segs == 1 ? i : i / segs;
+        const int w0 = kRecWords * (int)(i - r * segs);
         const float* x = Xb + r * Lg + gamma;
+        float v[kRecWords];
+#pragma unroll
+        for (int u = 0; u < kRecWords; ++u) {
+            const int c = 32 * (w0 + u) + lane;
+            v[u] = c < C ? x[4 * c] : 0.f;
+        }
+        unsigned mine = 0;
         bool any = false;
-        for (int w = 0; w < words; ++w) {
-            const int c = 32 * w + lane;
-            const float v = c < C ? x[4 * c] : 0.f;
-            if (c < C) codes[r * C + c] = v;
-            const unsigned b = __ballot_sync(0xffffffffu, c < C && v > thresh);
-            if (lane == 0) mask[r * words + w] = b;
+#pragma unroll
+        for (int u = 0; u < kRecWords; ++u) {
+            const int c = 32 * (w0 + u) + lane;
+            if (c < C) codes[r * C + c] = v[u];
+            const unsigned b = __ballot_sync(0xffffffffu, c < C && v[u] > thresh);
+            if (lane == u) mine = b;
             any |= b != 0;
         }
+        if (lane < kRecWords && w0 + lane < words) mask[r * words + w0 + lane] = mine;
         const int m = (int)(r % M);
         if (any && lane == 0 && !anym[m]) atomicOr(&anym[m], 1);
     }
@@ -263,8 +277,10 @@ int cdlgb_ar_create(int32_t N, int32_t L, int32_t M, int32_t T, int32_t device, 
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&a->stream, cudaStreamNonBlocking);
     size_t kcap = (size_t)T * M;
-    if (e == cudaSuccess) e = cudaMalloc((void**)&a->codes, (size_t)T * N * M * L * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&a->mask, (size_t)T * N * M * ((L + 31) / 32) * sizeof(unsigned));
+    // the codes and, in the same block (an allocation less: 20 us), their masks
+    const size_t rows = (size_t)T * N * M;
+    if (e == cudaSuccess) e = cudaMalloc((void**)&a->codes, rows * L * sizeof(float) + rows * ((L + 31) / 32) * sizeof(unsigned));
+    if (e == cudaSuccess) a->mask = reinterpret_cast<unsigned*>(a->codes + rows * L);
     if (e == cudaSuccess) e = cudaMalloc((void**)&a->anym, M * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc((void**)&a->kmap, kcap * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc((void**)&a->klen, kcap * sizeof(int));
@@ -281,8 +297,7 @@ int cdlgb_ar_destroy(cdlgb_ar* a) {
     if (!a) return CDLGB_OK;
     cudaSetDevice(a->dev);
     if (a->stream) cudaStreamSynchronize(a->stream);
-    void* ptrs[] = {a->codes, a->mask, a->anym, a->kmap, a->klen, a->dcount,
-                    a->msa};
+    void* ptrs[] = {a->codes, a->anym, a->kmap, a->klen, a->dcount, a->msa};
     for (void* p : ptrs) if (p) cudaFree(p);
     if (a->stream) cudaStreamDestroy(a->stream);
     delete a;
@@ -313,7 +328,7 @@ int cdlgb_ar_record(cdlgb_ar* a, cdlgb_ctx* c, double thresh, int32_t train_num,
     const float* Xb = c->best_is_cur ? c->Xb[c->xcur] : c->Xb[1 - c->xcur];
     AR_CU(a, cudaMemsetAsync(a->anym, 0, a->M * sizeof(int), a->stream));
     const size_t rows = (size_t)a->N * a->M, words = (a->C + 31) / 32;
-    k_record<<<grid_for(rows, 8), 256, 0, a->stream>>>(Xb, a->codes + t * rows * a->C, a->mask + t * rows * words,
+    k_record<<<grid_for(rows * ((words + kRecWords - 1) / kRecWords), 8), 256, 0, a->stream>>>(Xb, a->codes + t * rows * a->C, a->mask + t * rows * words,
                                                        rows, a->M, a->C, c->Lg, c->gamma, th, a->anym);
     AR_CU(a, cudaGetLastError());
     std::vector<int> any(a->M);
