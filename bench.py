@@ -310,6 +310,23 @@ def measured_hbm_peak() -> float:
         return 6800.0
 
 
+def xstep_kernel(Lg: int, M: int, fused: bool, steps_per_launch: int) -> str:
+    """What the X-step's timer covers, as far as the timers tell: the forms with a launch
+    per X-step are not told apart but on the headline sizes, where the convolution
+    form is not taken."""
+    if fused and steps_per_launch > 1:
+        shape = "<32, 29, 288, 1, 16>" if (Lg, M) == (928, 64) else ""
+        return (f"multi-iteration fused X-step k_xiter{shape} "
+                f"({steps_per_launch} X-steps per launch, duals on chip)")
+    if fused and (Lg, M) == (928, 64):
+        return "fused X-step kernel (k_xstep_warp<32, 29>, register-resident four-step FFTs)"
+    if fused:
+        return ("X-step (short convolutions: k_xc_codes + k_xc_solve, or k_xc_all; else in-kernel "
+                "FFTs: k_xstep_warp or k_xstep_fused)")
+    return ("X-step (short convolutions: k_xc_codes + k_xc_solve, or k_xc_all; else cuFFT path: "
+            "k_xprep + R2C + k_xsolve + C2R + k_mask_update)")
+
+
 def roofline(prof, steps, fused, sm_mhz=None):
     """Roofline of the dominant kernel, from the phase timers recorded (CUDA events on
     the launching stream) during the timed region.  For the multi-iteration X-step also
@@ -334,8 +351,6 @@ def roofline(prof, steps, fused, sm_mhz=None):
         ms_avg = prof["xfused"][0] / launches
         alg = ab["xstep"] * steps_per_launch
         if steps_per_launch > 1:
-            kernel = (f"multi-iteration fused X-step k_xiter<32, 29, 288, 1, 16> "
-                      f"({steps_per_launch} X-steps per launch, duals on chip)")
             if ab["Lg"] == 928 and WORKLOAD["M"] == 64:
                 # dram__bytes_read.sum + dram__bytes_write.sum of one launch (15 X-steps)
                 # captured by ncu on 1000 sequences, scaled per sequence
@@ -344,13 +359,13 @@ def roofline(prof, steps, fused, sm_mhz=None):
                     "pass over it, far below the per-X-step algorithmic bytes; the kernel is "
                     "bound by SM issue (FP32 FFT work), not HBM")
         else:
-            kernel = "fused X-step kernel (k_xstep_warp<32, 29>, register-resident four-step FFTs)"
             if ab["Lg"] == 928 and WORKLOAD["M"] == 64:
                 traffic = int(XWARP_DRAM_BYTES_N1000 / 1000 * WORKLOAD["N"])
     else:
         ms_avg = prof["xstep"][0] / max(prof["xstep"][1], 1)
         alg = ab["xstep"]
-        kernel = "X-step (cuFFT path: k_xprep + R2C + k_xsolve + C2R + k_mask_update)"
+        steps_per_launch = 1
+    kernel = xstep_kernel(ab["Lg"], WORKLOAD["M"], fused and prof["xfused"][1] > 0, steps_per_launch)
     achieved = alg / (ms_avg / 1e3) / 1e9
     out = {"bound": "hbm", "kernel": kernel, "achieved": round(achieved, 1), "peak": peak,
            "peak_source": peak_src, "unit": "GB/s", "frac": round(achieved / peak, 4),
@@ -556,7 +571,9 @@ def run_lengths(args, shapes=((100, 16), (200, 16), (500, 16), (200, 4)), N: int
     iterations after one untimed: outer iterations/s, the X-step and D-step device time
     per outer iteration from the library's phase timers, and the kernel path each length
     takes (register-FFT lengths run the multi-iteration X-step and the spectral D-step
-    on the register-FFT transforms; the others the generic in-kernel FFT X-step).  The
+    on the register-FFT transforms; the others, and those with few filters, the X-step
+    by short convolutions, and the D-step's rows on cuFFT where there is no register
+    FFT).  The
     X-step's and D-step's algorithmic bytes over their time give each one's HBM rate."""
     import torch
     pkg = _pkg()

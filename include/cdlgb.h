@@ -71,8 +71,11 @@ typedef struct {
     int32_t device;             /* CUDA device ordinal (default 0) */
     int32_t init_mode;          /* D0 == NULL: 0 = random normal, unit norm per filter;
                                    1 = the reference's simplex-per-base draw */
-    int32_t fft_mode;           /* 0 = auto (fused in-kernel FFT path where the size is
-                                   supported, else cuFFT transforms), 1 = cuFFT, 2 = fused */
+    int32_t fft_mode;           /* X-step: 0 = auto (the multi-iteration register-FFT kernel
+                                   where the size has one and M fills it, else short
+                                   convolutions, past 64 taps or Lg = 4128 only where they
+                                   are the cheaper form, else in-kernel FFTs or cuFFT),
+                                   1 = cuFFT, 2 = fused in-kernel FFTs */
     uint64_t hbm_budget_bytes;  /* 0 = free device memory minus a 1 GiB margin */
     float stop_tol;             /* stopping test of cdlgb_run_outer (no counterpart in the
                                    reference, whose loop count is fixed, wrap.jl:6-11):
