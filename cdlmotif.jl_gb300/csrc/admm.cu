@@ -681,9 +681,10 @@ int chunk_for(int N, int M, int Lg) {
     return (int)ch;
 }
 
-// Sequences per chunk of the spectral D-step: its only scratch is the Y3 half-spectra
-// (M x F complex per sequence), so a chunk covers up to 6 GB of them (the whole dataset
-// at N = 20000, L = 200, K = 64), never fewer than the cuFFT passes' chunk.
+// Sequences per chunk of the spectral D-step: its only scratch is the Y3 spectra, with
+// room for a half-spectrum of M x F complex values per sequence (the kept rows' spectra
+// that are stored take Lg/8 + 1 of the F), so a chunk covers up to 6 GB of them (the whole
+// dataset at N = 20000, L = 200, K = 64), never fewer than the cuFFT passes' chunk.
 int spec_chunk_for(int N, int M, int Lg) {
     size_t F = Lg / 2 + 1;
     size_t ch = ((size_t)6 << 30) / ((size_t)M * F * 8);

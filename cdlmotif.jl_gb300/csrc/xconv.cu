@@ -834,7 +834,7 @@ static bool xconv_allowed(const cdlgb_ctx* c) {
 // 0), and where those slots are empty enough, 5.5 + 0.03 T ps per filter against 4.8 per slot.
 // It is the more exact form there (32 trainings of 16 sizes, after one outer iteration against
 // float64: DX 2 to 20 times nearer than by the transforms, codes 2 to 6) and mostly the faster
-// one; where it is not (0.79 to 0.95 of the transforms' speed: M = 8, 10 with W = 16 at L = 200;
+// one; where it is not (0.76 to 0.95 of the transforms' speed: M = 8, 10 with W = 16 at L = 200;
 // odd M at Lg = 496 and 928; M = 9 at Lg = 4096) the more exact one is kept.  Past those sizes
 // the cheaper one is taken, by estimates in ps per X-step and code value from 2300 measured
 // sizes (Lg = 40-12288, M = 1-256, T = 4-128, 2 to 6e7 code values; 15 X-steps each way).  The
