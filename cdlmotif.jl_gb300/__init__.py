@@ -525,8 +525,9 @@ def _hit_counts(positions) -> np.ndarray:
 
 
 def _columns(a: np.ndarray, keep: np.ndarray) -> np.ndarray:
-    """The kept motifs' columns of an array of this module's own, as a C-order array (take
-    is faster than a boolean column index, and needs no bounds checks here)."""
+    """The kept motifs' columns of an array with a column per motif, as a C-order array, or the
+    array itself where all are kept (take is faster than a boolean column index, and without
+    bounds checks faster still)."""
     return a if keep.all() else a.take(np.flatnonzero(keep), axis=1, mode="clip")
 
 
